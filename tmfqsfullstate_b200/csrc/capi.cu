@@ -322,11 +322,19 @@ void copy_out(tmfqs_gpu_state *h, uint64_t first, double *host, uint64_t count) 
 	h->stats.d2h_bytes += count * 16;
 }
 
-tqb::SeqResult reduce(tmfqs_gpu_state *h, tqb::TermKind kind, const tqb::Overlay &ov, bool stop, double rnd) {
+tqb::SeqResult reduce(tmfqs_gpu_state *h, const tqb::Overlay &ov, bool stop, double rnd) {
 	flush_dirty(h);
-	h->stats.reduction_passes += 2;
-	PassTimer timer(h, TMFQS_KT_REDUCE, sweep_bytes(h));  // two read passes = one sweep's bytes
-	return tqb::seq_replay(h->precision, h->amps, h->N, kind, ov, stop, rnd, h->seq, h->stream, h->num_sms,
+	++h->stats.reduction_passes;
+	PassTimer timer(h, TMFQS_KT_REDUCE, sweep_bytes(h) / 2.0);  // one read
+	return tqb::seq_replay(h->precision, h->amps, h->N, ov, stop, rnd, h->seq, h->stream, h->num_sms,
+	                       &h->stats.kernel_launches);
+}
+
+void reduce_amplitudes(tmfqs_gpu_state *h, const tqb::Overlay &ov, double &re, double &im) {
+	flush_dirty(h);
+	++h->stats.reduction_passes;
+	PassTimer timer(h, TMFQS_KT_REDUCE, sweep_bytes(h) / 2.0);  // one read
+	tqb::seq_amplitude_sum(h->precision, h->amps, h->N, ov, re, im, h->seq, h->stream, h->num_sms,
 	                       &h->stats.kernel_launches);
 }
 
@@ -725,9 +733,9 @@ Cx logical_sum(tmfqs_gpu_state *h, const tmfqs_register_view &v) {
 	ov.sim = v.scale_im;
 	ov.bre = v.bias_re;
 	ov.bim = v.bias_im;
-	const double re = reduce(h, tqb::kTermReal, ov, false, 0.0).value;
-	const double im = reduce(h, tqb::kTermImag, ov, false, 0.0).value;
-	return {re, im};
+	Cx sum{0.0, 0.0};
+	reduce_amplitudes(h, ov, sum.re, sum.im);
+	return sum;
 }
 
 // Device value a float-stored state holds after `tr - v` in float.
@@ -1815,7 +1823,7 @@ int tmfqs_gpu_total_probability(tmfqs_gpu_state *h, double *out) {
 	return guarded([&] {
 		ensure_initialized(h, "total probability query");
 		DeviceScope d(h);
-		*out = reduce(h, tqb::kTermProb, tqb::Overlay{}, false, 0.0).value;
+		*out = reduce(h, tqb::Overlay{}, false, 0.0).value;
 	});
 }
 
@@ -1824,7 +1832,7 @@ int tmfqs_gpu_sample(tmfqs_gpu_state *h, double rnd, uint64_t *out) {
 		ensure_initialized(h, "measurement");
 		if(!(rnd >= 0.0 && rnd < 1.0)) fail(TMFQS_ERR_INVALID_ARGUMENT, "GpuStateBackend::sampleMeasurement requires rnd in [0,1)");
 		DeviceScope d(h);
-		const tqb::SeqResult r = reduce(h, tqb::kTermProb, tqb::Overlay{}, true, rnd);
+		const tqb::SeqResult r = reduce(h, tqb::Overlay{}, true, rnd);
 		if(r.index >= h->N) fail(TMFQS_ERR_RUNTIME, "GpuStateBackend::sampleMeasurement cumulative probability did not reach sample");
 		*out = r.index;
 	});
@@ -1834,8 +1842,7 @@ int tmfqs_gpu_amplitude_sum(tmfqs_gpu_state *h, double *re, double *im) {
 	return guarded([&] {
 		ensure_initialized(h, "amplitude sum");
 		DeviceScope d(h);
-		*re = reduce(h, tqb::kTermReal, tqb::Overlay{}, false, 0.0).value;
-		*im = reduce(h, tqb::kTermImag, tqb::Overlay{}, false, 0.0).value;
+		reduce_amplitudes(h, tqb::Overlay{}, *re, *im);
 	});
 }
 
@@ -1843,9 +1850,7 @@ int tmfqs_gpu_overlay_sum(tmfqs_gpu_state *h, double sre, double sim, double bre
 	return guarded([&] {
 		ensure_initialized(h, "amplitude sum");
 		DeviceScope d(h);
-		const tqb::Overlay ov{true, sre, sim, bre, bim};
-		*re = reduce(h, tqb::kTermReal, ov, false, 0.0).value;
-		*im = reduce(h, tqb::kTermImag, ov, false, 0.0).value;
+		reduce_amplitudes(h, tqb::Overlay{true, sre, sim, bre, bim}, *re, *im);
 	});
 }
 
@@ -1853,7 +1858,7 @@ int tmfqs_gpu_overlay_total_probability(tmfqs_gpu_state *h, double sre, double s
 	return guarded([&] {
 		ensure_initialized(h, "probability summation");
 		DeviceScope d(h);
-		*out = reduce(h, tqb::kTermProb, tqb::Overlay{true, sre, sim, bre, bim}, false, 0.0).value;
+		*out = reduce(h, tqb::Overlay{true, sre, sim, bre, bim}, false, 0.0).value;
 	});
 }
 
@@ -1861,7 +1866,7 @@ int tmfqs_gpu_overlay_sample(tmfqs_gpu_state *h, double sre, double sim, double 
 	return guarded([&] {
 		ensure_initialized(h, "measurement");
 		DeviceScope d(h);
-		const tqb::SeqResult r = reduce(h, tqb::kTermProb, tqb::Overlay{true, sre, sim, bre, bim}, true, rnd);
+		const tqb::SeqResult r = reduce(h, tqb::Overlay{true, sre, sim, bre, bim}, true, rnd);
 		if(r.index >= h->N) fail(TMFQS_ERR_RUNTIME, "QuantumRegister::measure cumulative probability did not reach sample");
 		*out = r.index;
 	});
@@ -1899,8 +1904,8 @@ int tmfqs_gpu_inversion(tmfqs_gpu_state *h) {
 	return guarded([&] {
 		ensure_initialized(h, "inversion about mean");
 		DeviceScope d(h);
-		const double sr = reduce(h, tqb::kTermReal, tqb::Overlay{}, false, 0.0).value;
-		const double si = reduce(h, tqb::kTermImag, tqb::Overlay{}, false, 0.0).value;
+		double sr = 0.0, si = 0.0;
+		reduce_amplitudes(h, tqb::Overlay{}, sr, si);
 		const double N = (double)h->N;
 		before_mutation(h);
 		{
@@ -2084,9 +2089,9 @@ int tmfqs_gpu_compare(tmfqs_gpu_state *ref, tmfqs_gpu_state *got, tmfqs_state_co
 		tqb::CompareReport r{};
 		tqb::launch_compare(ctx(ref), ref->precision, ref->amps, got->precision, got->amps, ref->N, r);
 		const tqb::Overlay none;
-		const double ref_sq = tqb::seq_replay(ref->precision, ref->amps, ref->N, tqb::kTermProb, none, false, 0.0, ref->seq,
+		const double ref_sq = tqb::seq_replay(ref->precision, ref->amps, ref->N, none, false, 0.0, ref->seq,
 		                                      ref->stream, ref->num_sms, &ref->stats.kernel_launches).value;
-		const double got_sq = tqb::seq_replay(got->precision, got->amps, got->N, tqb::kTermProb, none, false, 0.0, got->seq,
+		const double got_sq = tqb::seq_replay(got->precision, got->amps, got->N, none, false, 0.0, got->seq,
 		                                      got->stream, got->num_sms, &got->stats.kernel_launches).value;
 		const double diff_sq = tqb::seq_diff_norm(ref->precision, ref->amps, got->precision, got->amps, ref->N, ref->seq,
 		                                          ref->stream, ref->num_sms, &ref->stats.kernel_launches);

@@ -35,7 +35,7 @@ void arm_alloc_failures(unsigned skip, unsigned count);
 // ---------------------------------------------------------------------------
 // Exact sequential-sum engine (seqsum.cu)
 // ---------------------------------------------------------------------------
-enum TermKind { kTermProb = 0, kTermReal = 1, kTermImag = 2 };
+enum TermKind { kTermProb = 0, kTermAmp = 1 };
 
 struct Overlay {
 	bool active = false;
@@ -43,13 +43,9 @@ struct Overlay {
 };
 
 struct SeqScratch {
-	void *base = nullptr;  // one device allocation, carved below
+	void *base = nullptr;  // one device allocation
 	size_t bytes = 0;
-	uint64_t tiles = 0, groups = 0;
-	void *tile_a = nullptr, *tile_pre = nullptr, *tile_b = nullptr;
-	void *group_a = nullptr, *group_pre = nullptr, *group_b = nullptr;
-	void *walk_out = nullptr;  // WalkOut
-	void *host_out = nullptr;  // pinned WalkOut mirror
+	void *host_out = nullptr;  // pinned results
 };
 
 struct SeqResult {
@@ -57,10 +53,13 @@ struct SeqResult {
 	double value;    // running sum at that index (or the full sum)
 };
 
-// Computes the reference's left-to-right double sum of term(j), j < N, or
-// with stop=true the first j whose running sum reaches rnd.  Synchronises.
-SeqResult seq_replay(int precision, const void *amps, uint64_t N, TermKind kind, const Overlay &ov, bool stop,
-                     double rnd, SeqScratch &scratch, cudaStream_t stream, int num_sms, uint64_t *launches);
+// Computes the reference's left-to-right double sum of |a_j|^2, j < N, or with
+// stop=true the first j whose running sum reaches rnd.  Synchronises.
+SeqResult seq_replay(int precision, const void *amps, uint64_t N, const Overlay &ov, bool stop, double rnd,
+                     SeqScratch &scratch, cudaStream_t stream, int num_sms, uint64_t *launches);
+// The left-to-right sums of the real and the imaginary parts, from one read.  Synchronises.
+void seq_amplitude_sum(int precision, const void *amps, uint64_t N, const Overlay &ov, double &re, double &im,
+                       SeqScratch &scratch, cudaStream_t stream, int num_sms, uint64_t *launches);
 void seq_scratch_free(SeqScratch &scratch);
 // The reference's left-to-right sum over j of |got_j - ref_j|^2
 // (experiment::compareStates), exactly.  Synchronises.
