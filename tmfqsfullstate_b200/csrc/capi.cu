@@ -506,7 +506,7 @@ struct Planner {
 			                          tqb::launch_radix_pass(ctx(h), h->precision, h->amps, pass, h->dev_prog, h->dev_prog_bytes,
 			                                                 mirror));
 			mirrored = !qft && done && mirror;
-			if(!done) tqb::launch_fused_pass(ctx(h), h->precision, h->amps, pass, h->dev_prog, h->dev_prog_bytes);
+			if(!done) tqb::launch_fused_pass(ctx(h), h->precision, !twiddle, h->amps, pass, h->dev_prog, h->dev_prog_bytes);
 			++h->stats.fused_passes;
 		}
 	}
@@ -1264,7 +1264,7 @@ void load_apply_ops_body(tmfqs_gpu_state *h, unsigned n, const double *host, con
 		fp.tile_begin = v * per;
 		fp.tile_end = (v + 1) * per;
 		PassTimer timer(h, TMFQS_KT_FUSED, sweep_bytes(h) / slabs);
-		tqb::launch_fused_pass(ctx(h), h->precision, h->amps, fp, h->dev_prog, h->dev_prog_bytes);
+		tqb::launch_fused_pass(ctx(h), h->precision, true, h->amps, fp, h->dev_prog, h->dev_prog_bytes);
 	}
 	h->stats.h2d_bytes += h->N * 16;
 	++h->stats.fused_passes;

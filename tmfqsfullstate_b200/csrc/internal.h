@@ -170,10 +170,15 @@ struct FusedPass {
 	bool program_ready = false;
 };
 
-// Runs one fused pass over the whole state.  `dev_prog` is a device buffer
-// the launcher may (re)use for the program.
-void launch_fused_pass(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
+// Runs one fused pass over the whole state, with the reference's rounding when
+// `exact` (complex128 only).  `dev_prog` is a device buffer the launcher may
+// (re)use for the program.
+void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
                        size_t &dev_prog_bytes);
+// Any fused pass on a full tile as register stages (gate_pass.cu); false
+// (nothing launched) when its plan does not fit.
+bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
+                      size_t &dev_prog_bytes);
 
 // Uploads the program of an exact register-stage pass into `dev_prog` ahead
 // of its launches (the tile ranges of one pass share it); false when the pass
