@@ -341,6 +341,8 @@ void reduce_amplitudes(tmfqs_gpu_state *h, const tqb::Overlay &ov, double &re, d
 // ---------------------------------------------------------------------------
 // Fusion planner for tmfqs_gpu_apply_ops (the Simulator's gate runs).
 // ---------------------------------------------------------------------------
+void run_gate(tmfqs_gpu_state *h, const double *matrix, const unsigned *qubits, unsigned k);
+
 struct Planner {
 	tmfqs_gpu_state *h;
 	unsigned K;     // local bits of a pass
@@ -349,6 +351,8 @@ struct Planner {
 	uint64_t tmask = 0;  // bits that must be local (moving bits of ops in the pass)
 	int chain_op = -1;   // index of the H-chain op that may still grow
 	size_t nontrivial = 0;
+	unsigned ndense = 0;  // dense gates in the pass
+	unsigned Kfull;       // local bits of a full tile
 	std::vector<const tmfqs_op *> pending;  // circuit ops in the pass (for single-op fallback)
 	std::vector<unsigned> msched;  // fast forms: low-bit width of the first multi-op passes
 	unsigned mrest = 0;            // ... and of the passes after them
@@ -368,6 +372,7 @@ struct Planner {
 		// passes copy 16-byte granules and take rows of 32 (complex128) or 64
 		// (complex64) bytes, which leaves more bits per pass for the circuit.
 		const unsigned Kmax = h->precision == TMFQS_FP64 ? 12u : 13u;
+		Kfull = Kmax;
 		const bool fast = !h->opt_exact || h->precision == TMFQS_FP32;
 		if(fast && h->opt_radix) {
 			// Wider rows (up to four times the narrowest) stream far better when
@@ -409,8 +414,16 @@ struct Planner {
 		tmask = 0;
 		chain_op = -1;
 		nontrivial = 0;
+		ndense = 0;
 		pending.clear();
 	}
+
+	// Dense gates of one and two qubits join the passes of full tiles.  An exact
+	// two-qubit gate costs 30 us of FP64 work on 2^24 amplitudes, the pass 80 us
+	// of HBM traffic: from four on nothing is left to share.
+	bool takes_dense(unsigned k) const { return (k == 1 || k == 2) && K == Kfull && (!exact_form() || mlow >= 3); }
+	bool exact_form() const { return h->precision == TMFQS_FP64 && h->opt_exact; }
+	static constexpr unsigned kMaxDense = 4, kMaxDenseFast = 16;
 
 	// Whether bits in `m` can be local together with the current ones.
 	bool fits(uint64_t m) const {
@@ -485,7 +498,8 @@ struct Planner {
 				if(op.kind == tqb::kFH || op.kind == tqb::kFHChain || op.kind == tqb::kFHTwiddle || op.kind == tqb::kFX ||
 				   op.kind == tqb::kFCnot)
 					op.lt = local_index(op.lt);
-				if(op.kind == tqb::kFSwap) {
+				if(op.kind == tqb::kFDense1) op.lt = local_index(op.lt);
+				if(op.kind == tqb::kFSwap || op.kind == tqb::kFDense2) {
 					op.lt = local_index(op.lt);
 					op.lc = local_index(op.lc);
 				}
@@ -512,6 +526,7 @@ struct Planner {
 	}
 
 	void run_single(const tmfqs_op &op) {
+		if(op.kind == TMFQS_OP_GATE) return run_gate(h, op.matrix, op.qubits, op.k);
 		const auto c = ctx(h);
 		PassTimer timer(h, TMFQS_KT_GATE, sweep_bytes(h));
 		switch(op.kind) {
@@ -547,7 +562,27 @@ struct Planner {
 	}
 
 	void add(const tmfqs_op &op) {
+		// A pass with dense gates has no other kernel than the register stages,
+		// whose plan holds any 60 operations.
+		if(ndense && pending.size() >= 60) flush();
 		switch(op.kind) {
+			case TMFQS_OP_GATE: {
+				uint64_t m = 0;
+				for(unsigned i = 0; i < op.k; ++i) m |= 1ull << bit_of(h, op.qubits[i]);
+				if(!fits(m) || pending.size() >= 60 || ndense >= (exact_form() ? kMaxDense : kMaxDenseFast)) flush();
+				tmask |= m;
+				tqb::FusedOp f{};
+				f.kind = op.k == 1 ? tqb::kFDense1 : tqb::kFDense2;
+				f.lt = bit_of(h, op.qubits[0]);
+				if(op.k == 2) f.lc = bit_of(h, op.qubits[1]);
+				f.tab = (uint32_t)pass.mats.size();
+				pass.mats.insert(pass.mats.end(), op.matrix, op.matrix + (size_t(2) << (2 * op.k)));
+				pass.ops.push_back(f);
+				pending.push_back(&op);
+				++ndense;
+				chain_op = -1;
+				return;
+			}
 			case TMFQS_OP_H: add_pair_op(op, tqb::kFH, bit_of(h, op.q0), 0); return;
 			case TMFQS_OP_X: add_pair_op(op, tqb::kFX, bit_of(h, op.q0), 0); return;
 			case TMFQS_OP_CNOT: add_pair_op(op, tqb::kFCnot, bit_of(h, op.q1), 1ull << bit_of(h, op.q0)); return;
@@ -660,7 +695,7 @@ void run_gate(tmfqs_gpu_state *h, const double *matrix, const unsigned *qubits, 
 	for(unsigned i = 0; i < k; ++i) tpos[i] = bit_of(h, qubits[i]);
 	{
 		PassTimer timer(h, TMFQS_KT_GATE, sweep_bytes(h));
-		tqb::launch_gate(ctx(h), h->precision, h->amps, h->n, k, static_cast<const double *>(h->dev_small), tpos.data());
+		tqb::launch_gate(ctx(h), h->precision, h->opt_exact, h->amps, h->n, k, static_cast<const double *>(h->dev_small), tpos.data());
 	}
 	check_cuda(cudaStreamSynchronize(h->stream), "gate sync");
 	++h->stats.gate_passes;
@@ -969,6 +1004,11 @@ size_t dense_block_extent(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, siz
 	for(; j < count; ++j) {
 		std::vector<unsigned> qs;
 		std::vector<std::complex<double>> g;
+		try {
+			validate_op(h, ops[j]);
+		} catch(const tqb::Error &) {
+			break;  // the ops before an invalid one are applied, then it is reported
+		}
 		if(!op_as_matrix(ops[j], qs, g)) break;
 		std::vector<unsigned> U = Q;
 		for(unsigned q : qs)
@@ -978,6 +1018,25 @@ size_t dense_block_extent(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, siz
 		has_gate = has_gate || ops[j].kind == TMFQS_OP_GATE;
 	}
 	return j;
+}
+
+// Whether the run of ops starting at ops[i] within 5 qubits is applied as one
+// block sweep.  Gates of one and two qubits do better in the fused passes,
+// which hold gates on 9 to 11 qubits (two-qubit gates on 2^27 complex64
+// amplitudes: about 60 us each there, a block sweep 515 us whatever it holds),
+// unless the block is the whole rest of the batch, or holds many of them.
+bool block_wanted(tmfqs_gpu_state *h, const Planner &p, const tmfqs_op *ops, size_t i, size_t count) {
+	bool has_gate = false;
+	const size_t jend = dense_block_extent(h, ops, i, count, has_gate);
+	if(!has_gate || jend - i < 2) return false;
+	if(!p.takes_dense(2)) return true;
+	unsigned gates = 0, wide = 0;
+	for(size_t j = i; j < jend; ++j)
+		if(ops[j].kind == TMFQS_OP_GATE) {
+			++gates;
+			wide += ops[j].k > 2;
+		}
+	return wide || gates >= 8 || (p.pending.empty() && jend == count);
 }
 
 // Starting at ops[i], the longest run of ops acting within 5 qubits (holding
@@ -1101,6 +1160,8 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 	}
 	Planner p(h);
 	p.base = ops;
+	bool blocks = false;
+	for(size_t j = 0; j < count && !blocks; ++j) blocks = block_fusion(h) && ops[j].kind == TMFQS_OP_GATE;
 	size_t i = 0;
 	try {
 		while(i < count) {
@@ -1124,33 +1185,25 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 					continue;
 				}
 			}
-			if(op.kind == TMFQS_OP_GATE) {
+			// A dense gate, or gates that lead into one, and the ops after it
+			// that stay within 5 qubits: one block sweep.
+			if(blocks && block_wanted(h, p, ops, i, count)) {
 				p.flush();
 				h->cur_first = i;
 				h->cur_count = 1;
-				// A dense gate and the ops after it that stay within 5 qubits: one block sweep.
 				const size_t used = run_dense_block(h, ops, i, count);
 				if(used) {
 					i += used;
 					continue;
 				}
+			}
+			if(op.kind == TMFQS_OP_GATE && !p.takes_dense(op.k)) {
+				p.flush();
+				h->cur_first = i;
+				h->cur_count = 1;
 				run_gate(h, op.matrix, op.qubits, op.k);
 				++i;
 				continue;
-			}
-			if(block_fusion(h)) {
-				// Gates that lead into a dense gate within the same 5 qubits join its block.
-				bool has_gate = false;
-				const size_t jend = dense_block_extent(h, ops, i, count, has_gate);
-				if(has_gate && jend - i >= 2) {
-					validate_op(h, op);
-					p.flush();
-					const size_t used = run_dense_block(h, ops, i, count);
-					if(used) {
-						i += used;
-						continue;
-					}
-				}
 			}
 			p.add(op);
 			++i;

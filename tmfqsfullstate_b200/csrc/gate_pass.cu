@@ -1,7 +1,8 @@
 // General fused passes as register stages: any mix of Hadamards, X, CNOTs,
-// swaps, controlled phases and basis-state flips on a tile's local bits.
+// swaps, dense one- and two-qubit gates, controlled phases and basis-state flips
+// on a tile's local bits.
 //
-// A pass's moving operations (H, X, CNOT) are cut, in circuit order, into stages
+// A pass's moving operations (H, X, CNOT, dense gates) are cut, in circuit order, into stages
 // of up to four distinct targets.  In a stage every thread holds the 16
 // amplitudes of the tile that differ in the stage's four register bits and
 // applies the stage's operations to them in registers; diagonal operations run
@@ -21,6 +22,9 @@
 // operations on 23 qubits complex128 (41 us at the copy rate) takes 81-181 us, and
 // one of 10-21 on 26 qubits complex64 (164 us) 345-612 us; op by op through shared
 // memory with a barrier each (k_fused) they took 205-471 us and 900-1850 us.
+// Dense two-qubit gates are arithmetic: 30 us of FP64 each on 24 qubits exact (four
+// in a pass 235 us, alone 104 us each), 107 us each on 27 qubits complex64 (four in
+// a pass 750 us; as tensor-core blocks of two 515 us per block).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -36,7 +40,7 @@ namespace {
 constexpr unsigned kRB = 4;            // register bits per stage
 constexpr unsigned kRegs = 1u << kRB;  // amplitudes per thread
 constexpr unsigned kMaxK = 13;
-constexpr unsigned kMaxStages = 24;
+constexpr unsigned kMaxStages = 64;
 constexpr unsigned kMaxOps = 240;
 
 // Tiles of 64 KiB.
@@ -52,18 +56,19 @@ constexpr unsigned line_bits() {
 
 // Operation codes: kCodeH + register bit; kCodeX + 4 * target + control register
 // bit (the target itself: none); kCodeCP + mask of register bits that must be
-// set; kCodeFlip.
-constexpr unsigned kCodeH = 0, kCodeX = 4, kCodeCP = 20, kCodeFlip = 36;
+// set; kCodeFlip; kCodeU1 + register bit; kCodeU2 + 4 * first + second register
+// bit (the first is the more significant one of the gate's block index).
+constexpr unsigned kCodeH = 0, kCodeX = 4, kCodeCP = 20, kCodeFlip = 36, kCodeU1 = 37, kCodeU2 = 41;
 
 struct GateOp {
 	uint32_t code;
 	uint16_t tmask, rval;  // thread index bits that must be set; flips: the thread index and the register of the state
-	uint64_t omask;        // outer index bits that must be set; flips: the state's outer bits
+	uint64_t omask;        // outer index bits that must be set; flips: the state's outer bits; dense gates: the matrix
 	double cr, ci;
 };
 
 struct GateGeom {
-	unsigned n, nstages, nops;
+	unsigned n, nstages, nops, nmat;  // nmat: complex matrix elements of the dense gates
 	uint64_t o_begin, ntiles;  // the launch runs tiles [o_begin, ntiles)
 	double inv, scale;  // 1/sqrt(2); fast forms: the pass's power of it
 	uint64_t outer;     // mask of the index bits outside the tile
@@ -151,8 +156,77 @@ __device__ __forceinline__ void op_cp(typename Vec2<R>::type (&v)[kRegs], R pr, 
 	}
 }
 
+// Dense gate on register bit I: the unrolled formula of gate_block_apply.h:117-140.
+template <typename R, bool EXACT, unsigned I>
+__device__ __forceinline__ void op_u1(typename Vec2<R>::type (&v)[kRegs], const typename Vec2<R>::type *m) {
+	const auto g00 = m[0], g01 = m[1], g10 = m[2], g11 = m[3];
+#pragma unroll
+	for(unsigned r = 0; r < kRegs; ++r) {
+		if((r >> I) & 1u) continue;
+		const auto x = v[r], y = v[r | (1u << I)];
+		if constexpr(EXACT) {
+			if((nonzero_bits(x) | nonzero_bits(y)) == 0u) continue;
+			v[r].x = rsub(radd(rsub(rmul(g00.x, x.x), rmul(g00.y, x.y)), rmul(g01.x, y.x)), rmul(g01.y, y.y));
+			v[r].y = radd(radd(radd(rmul(g00.x, x.y), rmul(g00.y, x.x)), rmul(g01.x, y.y)), rmul(g01.y, y.x));
+			v[r | (1u << I)].x = rsub(radd(rsub(rmul(g10.x, x.x), rmul(g10.y, x.y)), rmul(g11.x, y.x)), rmul(g11.y, y.y));
+			v[r | (1u << I)].y = radd(radd(radd(rmul(g10.x, x.y), rmul(g10.y, x.x)), rmul(g11.x, y.y)), rmul(g11.y, y.x));
+		} else {
+			v[r].x = fma(-g01.y, y.y, fma(g01.x, y.x, fma(-g00.y, x.y, g00.x * x.x)));
+			v[r].y = fma(g01.y, y.x, fma(g01.x, y.y, fma(g00.y, x.x, g00.x * x.y)));
+			v[r | (1u << I)].x = fma(-g11.y, y.y, fma(g11.x, y.x, fma(-g10.y, x.y, g10.x * x.x)));
+			v[r | (1u << I)].y = fma(g11.y, y.x, fma(g11.x, y.y, fma(g10.y, x.x, g10.x * x.y)));
+		}
+	}
+}
+
+// A matrix element from shared memory, loaded where it is used: a broadcast,
+// and cheaper than the spills of keeping the whole matrix in registers.
+__device__ __forceinline__ double2 mat_at(const double2 *m) {
+	double2 x;
+	asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.x), "=d"(x.y) : "r"((unsigned)__cvta_generic_to_shared(m)));
+	return x;
+}
+__device__ __forceinline__ float2 mat_at(const float2 *m) {
+	float2 x;
+	asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"((unsigned)__cvta_generic_to_shared(m)));
+	return x;
+}
+
+// Dense gate on register bits A (more significant) and B: row sums term by term
+// (gate_block_apply.h:165-176); all-zero blocks are left alone.
+template <typename R, bool EXACT, unsigned A, unsigned B>
+__device__ __forceinline__ void op_u2(typename Vec2<R>::type (&v)[kRegs], const typename Vec2<R>::type *m) {
+#pragma unroll
+	for(unsigned r = 0; r < kRegs; ++r) {
+		if(((r >> A) & 1u) || ((r >> B) & 1u)) continue;
+		const unsigned at[4] = {r, r | (1u << B), r | (1u << A), r | (1u << A) | (1u << B)};
+		typename Vec2<R>::type o[4];
+		if constexpr(EXACT)
+			if((nonzero_bits(v[at[0]]) | nonzero_bits(v[at[1]]) | nonzero_bits(v[at[2]]) | nonzero_bits(v[at[3]])) == 0u) continue;
+#pragma unroll
+		for(unsigned row = 0; row < 4; ++row) {
+			R nr = R(0), ni = R(0);
+#pragma unroll
+			for(unsigned c = 0; c < 4; ++c) {
+				const auto g = mat_at(m + 4 * row + c), x = v[at[c]];
+				if constexpr(EXACT) {
+					nr = radd(nr, rsub(rmul(g.x, x.x), rmul(g.y, x.y)));
+					ni = radd(ni, radd(rmul(g.x, x.y), rmul(g.y, x.x)));
+				} else {
+					nr = fma(-g.y, x.y, fma(g.x, x.x, nr));
+					ni = fma(g.y, x.x, fma(g.x, x.y, ni));
+				}
+			}
+			o[row].x = nr;
+			o[row].y = ni;
+		}
+#pragma unroll
+		for(unsigned c = 0; c < 4; ++c) v[at[c]] = o[c];
+	}
+}
+
 template <typename R, bool EXACT>
-__device__ __forceinline__ void run_op(const GateOp &op, typename Vec2<R>::type (&v)[kRegs], const GateGeom &g, uint64_t base, unsigned t) {
+__device__ __forceinline__ void run_op(const GateOp &op, typename Vec2<R>::type (&v)[kRegs], const GateGeom &g, const typename Vec2<R>::type *mats, uint64_t base, unsigned t) {
 	if(op.code == kCodeFlip) {
 		const unsigned at = (base & g.outer) == op.omask && t == op.tmask ? op.rval : kRegs;
 #pragma unroll
@@ -161,6 +235,21 @@ __device__ __forceinline__ void run_op(const GateOp &op, typename Vec2<R>::type 
 			v[r].y = r == at ? -v[r].y : v[r].y;
 		}
 		return;
+	}
+	if(op.code >= kCodeU1) {
+		const typename Vec2<R>::type *m = mats + op.omask;
+		switch(op.code) {
+#define TQB_U1(I) \
+	case kCodeU1 + I: op_u1<R, EXACT, I>(v, m); return;
+#define TQB_U2(A, B) \
+	case kCodeU2 + 4 * A + B: op_u2<R, EXACT, A, B>(v, m); return;
+			TQB_U1(0) TQB_U1(1) TQB_U1(2) TQB_U1(3)
+			TQB_U2(0, 1) TQB_U2(0, 2) TQB_U2(0, 3) TQB_U2(1, 0) TQB_U2(1, 2) TQB_U2(1, 3)
+			TQB_U2(2, 0) TQB_U2(2, 1) TQB_U2(2, 3) TQB_U2(3, 0) TQB_U2(3, 1) TQB_U2(3, 2)
+#undef TQB_U1
+#undef TQB_U2
+			default: return;
+		}
 	}
 	if((base & op.omask) != op.omask) return;
 	const bool on = (t & op.tmask) == op.tmask;
@@ -200,15 +289,21 @@ __device__ __forceinline__ unsigned slot_of(unsigned b) {
 
 template <typename R, bool EXACT>
 __global__ void __launch_bounds__(1u << (tile_bits<R>() - kRB), 2) k_gate_pass(typename Vec2<R>::type *a, const __grid_constant__ GateGeom g,
-                                                                              const GateOp *gops) {
+                                                                              const GateOp *gops, const double2 *gmats) {
 	typedef typename Vec2<R>::type V;
 	constexpr unsigned K = tile_bits<R>(), TB = K - kRB;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	V *s = reinterpret_cast<V *>(smem_raw);
 	GateOp *ops = reinterpret_cast<GateOp *>(smem_raw + (sizeof(V) << K));
+	V *mats = reinterpret_cast<V *>(ops + g.nops);
 	const unsigned t = threadIdx.x;
 	for(unsigned e = t; e < g.nops * (sizeof(GateOp) / 16); e += blockDim.x)
 		reinterpret_cast<int4 *>(ops)[e] = reinterpret_cast<const int4 *>(gops)[e];
+	for(unsigned e = t; e < g.nmat; e += blockDim.x) {
+		const double2 x = gmats[e];
+		mats[e].x = (R)x.x;
+		mats[e].y = (R)x.y;
+	}
 	__syncthreads();
 	for(uint64_t o = g.o_begin + blockIdx.x; o < g.ntiles; o += gridDim.x) {
 		uint64_t base = o;
@@ -255,7 +350,7 @@ __global__ void __launch_bounds__(1u << (tile_bits<R>() - kRB), 2) k_gate_pass(t
 				for(unsigned r = 0; r < kRegs; ++r) v[r] = s[at(r)];
 			}
 			const unsigned k1 = (unsigned)g.first[st] + g.count[st];
-			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT>(ops[k], v, g, base, t);
+			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT>(ops[k], v, g, mats, base, t);
 			if(last) {
 				uint64_t go[kRB];
 				const uint64_t gb = global(g.opos, go);
@@ -284,8 +379,9 @@ __global__ void __launch_bounds__(1u << (tile_bits<R>() - kRB), 2) k_gate_pass(t
 // One operation of the pass on tile bits: `pm` the tile bits and `om` the outer
 // index bits that must be set.
 struct PlanOp {
-	enum Kind { kH, kX, kCP, kFlip } kind;
-	unsigned p;  // the moving tile bit
+	enum Kind { kH, kX, kCP, kFlip, kU1, kU2 } kind;
+	unsigned p, p2;  // the moving tile bit(s)
+	unsigned mat;    // dense gates: first element of the matrix
 	uint32_t pm;
 	uint64_t om;
 	double cr, ci;
@@ -363,6 +459,14 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 				require(q, op.state);
 				ops.push_back(q);
 				break;
+			case kFDense1:
+			case kFDense2:
+				q.kind = op.kind == kFDense1 ? PlanOp::kU1 : PlanOp::kU2;
+				q.p = where[op.lt];
+				if(op.kind == kFDense2) q.p2 = where[op.lc];
+				q.mat = op.tab / 2;
+				ops.push_back(q);
+				break;
 			case kFSwap: std::swap(where[op.lt], where[op.lc]); break;
 			default: return false;
 		}
@@ -378,16 +482,15 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 	std::vector<uint32_t> regs{0u};
 	std::vector<std::vector<unsigned>> of(1);
 	for(unsigned k = 0; k < ops.size(); ++k) {
-		if(ops[k].kind == PlanOp::kH || ops[k].kind == PlanOp::kX) {
-			const uint32_t bit = 1u << ops[k].p;
-			uint32_t &r = regs.back();
-			if(!(r & bit)) {
-				if(__builtin_popcount(r) == (int)kRB || (regs.size() == 1 && (keep_in & bit))) {
-					regs.push_back(bit);
-					of.push_back({});
-				} else {
-					r |= bit;
-				}
+		uint32_t bits = 0;
+		if(ops[k].kind != PlanOp::kCP && ops[k].kind != PlanOp::kFlip) bits = 1u << ops[k].p;
+		if(ops[k].kind == PlanOp::kU2) bits |= 1u << ops[k].p2;
+		if(bits & ~regs.back()) {
+			if(__builtin_popcount(regs.back() | bits) > (int)kRB || (regs.size() == 1 && (keep_in & bits))) {
+				regs.push_back(bits);
+				of.push_back({});
+			} else {
+				regs.back() |= bits;
 			}
 		}
 		of.back().push_back(k);
@@ -453,9 +556,11 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 			uint32_t rm = 0, tm = 0;
 			for(unsigned i = 0; i < kRB; ++i) rm |= ((q.pm >> rb[i]) & 1u) << i;
 			for(unsigned i = 0; i < tb.size(); ++i) tm |= ((q.pm >> tb[i]) & 1u) << i;
-			unsigned target = 0;
-			for(unsigned i = 0; i < kRB; ++i)
+			unsigned target = 0, second = 0;
+			for(unsigned i = 0; i < kRB; ++i) {
 				if(rb[i] == q.p) target = i;
+				if(rb[i] == q.p2) second = i;
+			}
 			o.tmask = (uint16_t)tm;
 			o.omask = q.om;
 			o.cr = q.cr;
@@ -468,11 +573,17 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 					o.code = kCodeFlip;
 					o.rval = (uint16_t)rm;
 					break;
+				case PlanOp::kU1:
+				case PlanOp::kU2:
+					o.code = q.kind == PlanOp::kU1 ? kCodeU1 + target : kCodeU2 + 4 * target + second;
+					o.omask = q.mat;
+					break;
 			}
 			out.push_back(o);
 		}
 	}
 	g.nops = (unsigned)out.size();
+	g.nmat = (unsigned)(pass.mats.size() / 2);
 	g.scale = std::pow(2.0, -0.5 * (double)nh);
 	return true;
 }
@@ -483,7 +594,8 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	GateGeom g;
 	std::vector<GateOp> ops;
 	if(!plan_gates(pass, K, line_bits<R>(), g, ops)) return false;
-	const size_t need = std::max<size_t>(1, ops.size()) * sizeof(GateOp);
+	const size_t ops_bytes = ops.size() * sizeof(GateOp), mat_bytes = pass.mats.size() * sizeof(double);
+	const size_t need = std::max<size_t>(sizeof(GateOp), ops_bytes + mat_bytes);
 	if(need > dev_prog_bytes) {
 		if(dev_prog) {
 			check_cuda(cudaStreamSynchronize(c.stream), "gate pass program sync");
@@ -497,15 +609,20 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 		}
 		dev_prog_bytes = need * 2;
 	}
-	if(!ops.empty()) upload_async(c, dev_prog, ops.data(), ops.size() * sizeof(GateOp), "gate pass program upload");
-	const size_t smem = (sizeof(typename Vec2<R>::type) << K) + ops.size() * sizeof(GateOp);
+	std::vector<unsigned char> host(need);
+	if(ops_bytes) std::memcpy(host.data(), ops.data(), ops_bytes);
+	if(mat_bytes) std::memcpy(host.data() + ops_bytes, pass.mats.data(), mat_bytes);
+	if(ops_bytes + mat_bytes) upload_async(c, dev_prog, host.data(), ops_bytes + mat_bytes, "gate pass program upload");
+	typedef typename Vec2<R>::type V;
+	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(V);
 	auto kern = k_gate_pass<R, EXACT>;
 	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gate pass smem");
 	const unsigned threads = 1u << (K - kRB);
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem), "gate pass occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));
-	kern<<<(unsigned)grid, threads, smem, c.stream>>>(static_cast<typename Vec2<R>::type *>(a), g, static_cast<const GateOp *>(dev_prog));
+	kern<<<(unsigned)grid, threads, smem, c.stream>>>(static_cast<V *>(a), g, static_cast<const GateOp *>(dev_prog),
+	                                                 reinterpret_cast<const double2 *>(static_cast<unsigned char *>(dev_prog) + ops_bytes));
 	check_cuda(cudaGetLastError(), "gate pass");
 	if(c.launches) ++*c.launches;
 	return true;

@@ -115,8 +115,9 @@ void launch_scatter_uniform(const LaunchCtx &c, int prec, void *a, const uint64_
 void launch_scatter_values(const LaunchCtx &c, int prec, void *a, const uint64_t *idx, const double *vals,
                            uint64_t count);
 // matrix: device, row-major 2^k x 2^k interleaved complex (double);
-// tpos: device array of the k target bit positions in block order.
-void launch_gate(const LaunchCtx &c, int prec, void *a, unsigned n, unsigned k, const double *matrix,
+// tpos: host array of the k target bit positions in block order.  exact: the
+// reference's rounding (complex128).
+void launch_gate(const LaunchCtx &c, int prec, bool exact, void *a, unsigned n, unsigned k, const double *matrix,
                  const unsigned *tpos_host);
 // complex128 <-> complex64 conversion of `count` amplitudes (device buffers).
 void launch_to_c64(const LaunchCtx &c, void *dst, const double *src, uint64_t count);
@@ -133,7 +134,9 @@ enum FusedOpKind : uint32_t {
 	kFCP = 4,      // controlled phase, any two bits (diagonal)
 	kFFlip = 5,    // phase flip of one basis state (diagonal)
 	kFSwap = 6,    // swap of two local bits
-	kFHTwiddle = 7 // Hadamard, then its H-chain applied as one twiddle per |1> output
+	kFHTwiddle = 7, // Hadamard, then its H-chain applied as one twiddle per |1> output
+	kFDense1 = 8,  // dense gate on local bit lt, matrix at FusedPass::mats[tab]
+	kFDense2 = 9   // dense gate on local bits lt (most significant) and lc
 };
 
 struct FusedOp {
@@ -162,6 +165,7 @@ struct FusedPass {
 	unsigned lpos[16] = {0};        // global bit position of local bit i, ascending
 	std::vector<FusedOp> ops;
 	std::vector<ChainEntry> chain;  // H-chain entries of all chains of the pass
+	std::vector<double> mats;       // matrices of the dense gates, row-major interleaved complex
 	unsigned gate_count = 0;        // circuit operations folded into this pass
 	// Exact fused passes: run only tiles [tile_begin, tile_end) (0, 0: all).
 	uint64_t tile_begin = 0, tile_end = 0;
