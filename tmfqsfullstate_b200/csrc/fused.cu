@@ -198,9 +198,12 @@ __global__ void __launch_bounds__(kFusedThreads, 3) k_fused(typename Vec2<R>::ty
 						} else {
 							// The other warps stage the op's layout in shared memory.
 							const ChainMap &gm = maps[op.state];
-							for(unsigned k = threadIdx.x - 32; k < gm.nq; k += blockDim.x - 32) {
-								smr[k] = gm.mr[k];
-								sjr[k] = gm.jr[k];
+							// (a thread takes kChainPairs of them at once: with fewer, as in
+							// tiles of 7 bits, the last ones again)
+							const unsigned nk = max(gm.nq, kChainPairs);
+							for(unsigned k = threadIdx.x - 32; k < nk; k += blockDim.x - 32) {
+								smr[k] = gm.mr[k & (gm.nq - 1u)];
+								sjr[k] = gm.jr[k & (gm.nq - 1u)];
 							}
 							if(threadIdx.x < 64) {
 								sml[threadIdx.x - 32] = gm.ml[threadIdx.x - 32];
