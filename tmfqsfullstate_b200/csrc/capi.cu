@@ -1169,8 +1169,17 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 			validate_op(h, op);
 			if(op.kind == TMFQS_OP_SWAP) {
 				const size_t run = swap_run(ops, i, count);
-				if(run >= 2) {
-					for(size_t j = i; j < i + run; ++j) validate_op(h, ops[j]);
+				// A swap of tile bits is free in a fused pass (it relabels them), the
+				// permutation a sweep of its own: short runs go into the passes, and so
+				// do longer ones whose bits the current pass holds anyway (exact form;
+				// the fast forms' QFT pass takes no swaps).
+				uint64_t m = 0;
+				for(size_t j = i; j < i + run; ++j) {
+					validate_op(h, ops[j]);
+					m |= (1ull << bit_of(h, ops[j].q0)) | (1ull << bit_of(h, ops[j].q1));
+				}
+				const bool in_pass = run < 4 || (p.exact_form() && p.fits(m));
+				if(!in_pass) {
 					p.flush();
 					std::vector<std::pair<unsigned, unsigned>> pairs;
 					for(size_t j = i; j < i + run; ++j) pairs.push_back({bit_of(h, ops[j].q0), bit_of(h, ops[j].q1)});

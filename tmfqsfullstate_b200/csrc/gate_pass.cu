@@ -3,9 +3,9 @@
 // on a tile's local bits.
 //
 // A pass's moving operations (H, X, CNOT, dense gates) are cut, in circuit order, into stages
-// of up to four distinct targets.  In a stage every thread holds the 16
-// amplitudes of the tile that differ in the stage's four register bits and
-// applies the stage's operations to them in registers; diagonal operations run
+// of up to four (complex64: five) distinct targets.  In a stage every thread
+// holds the 16 (32) amplitudes of the tile that differ in the stage's register
+// bits and applies the stage's operations to them in registers; diagonal operations run
 // in whatever stage they fall into, under per-thread and per-register
 // conditions.  The first stage reads the tile from HBM, the last writes it back,
 // those between pass it on through shared memory with one barrier each.  A swap
@@ -18,13 +18,16 @@
 // without their 1/sqrt(2), which is applied once as a power at the end.
 //
 // Bound: HBM (one read and one write per pass) and, behind it, instruction issue:
-// about 100 instructions per operation and 16 amplitudes.  A pass of 12-35 mixed
-// operations on 23 qubits complex128 (41 us at the copy rate) takes 81-181 us, and
-// one of 10-21 on 26 qubits complex64 (164 us) 345-612 us; op by op through shared
-// memory with a barrier each (k_fused) they took 205-471 us and 900-1850 us.
+// about 60 instructions per operation and 16 amplitudes, at half the issue rate
+// (16 warps per SM, one code path after another through the instruction caches).
+// A pass of 11-35 mixed operations on 23 qubits complex128 (41 us at the copy rate)
+// takes 77-167 us, and one of 10-21 on 26 qubits complex64 (164 us) 276-483 us; op
+// by op through shared memory with a barrier each (k_fused) 205-471 and 900-1850 us.
+// 32 complex64 amplitudes per thread against 16: 12% less; zero tests on the high
+// words first: 3%; dense gates in a kernel of their own: 9%.
 // Dense two-qubit gates are arithmetic: 30 us of FP64 each on 24 qubits exact (four
-// in a pass 235 us, alone 104 us each), 107 us each on 27 qubits complex64 (four in
-// a pass 750 us; as tensor-core blocks of two 515 us per block).
+// in a pass 230 us, alone 104 us each), 75 us each on 27 qubits complex64 (four in
+// a pass 660 us; as tensor-core blocks of two 515 us per block).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -37,10 +40,10 @@ namespace tqb {
 
 namespace {
 
-constexpr unsigned kRB = 4;            // register bits per stage
-constexpr unsigned kRegs = 1u << kRB;  // amplitudes per thread
+constexpr unsigned kMaxRB = 5;
 constexpr unsigned kMaxK = 13;
 constexpr unsigned kMaxStages = 64;
+constexpr unsigned kSlotStages = 8;  // stages whose thread slots are kept in shared memory
 constexpr unsigned kMaxOps = 240;
 
 // Tiles of 64 KiB.
@@ -48,17 +51,24 @@ template <typename R>
 constexpr unsigned tile_bits() {
 	return sizeof(R) == 8 ? 12u : 13u;
 }
+// Register bits per stage: 16 complex128 or 32 complex64 amplitudes per thread (64 registers), 256 threads.
+template <typename R>
+constexpr unsigned reg_bits() {
+	return sizeof(R) == 8 ? 4u : 5u;
+}
+constexpr unsigned kThreadBits = 8, kThreads = 1u << kThreadBits;
 // Index bits of a 128-byte line: lanes in stages that touch HBM, and the shared-memory slot bits that pick a bank group.
 template <typename R>
 constexpr unsigned line_bits() {
 	return sizeof(R) == 8 ? 3u : 4u;
 }
 
-// Operation codes: kCodeH + register bit; kCodeX + 4 * target + control register
+// Operation codes: kCodeH + register bit; kCodeX + 5 * target + control register
 // bit (the target itself: none); kCodeCP + mask of register bits that must be
-// set; kCodeFlip; kCodeU1 + register bit; kCodeU2 + 4 * first + second register
-// bit (the first is the more significant one of the gate's block index).
-constexpr unsigned kCodeH = 0, kCodeX = 4, kCodeCP = 20, kCodeFlip = 36, kCodeU1 = 37, kCodeU2 = 41;
+// set; kCodeFlip; kCodeU1 + register bit; kCodeU2 + 5 * first + second register
+// bit (the first is the more significant one of the gate's block index; in the
+// fast forms always the higher one).
+constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeFlip = 62, kCodeU1 = 63, kCodeU2 = 68;
 
 struct GateOp {
 	uint32_t code;
@@ -74,8 +84,8 @@ struct GateGeom {
 	uint64_t outer;     // mask of the index bits outside the tile
 	uint8_t lpos[kMaxK], opos[kMaxK];  // index bit of a tile bit when loaded and when stored
 	uint8_t first[kMaxStages], count[kMaxStages];
-	uint8_t rbit[kMaxStages][kRB];          // tile bit of register bit i
-	uint8_t tbit[kMaxStages][kMaxK - kRB];  // tile bit of thread index bit k
+	uint8_t rbit[kMaxStages][kMaxRB];        // tile bit of register bit i
+	uint8_t tbit[kMaxStages][kThreadBits];  // tile bit of thread index bit k
 };
 
 // Non-sign bits of an amplitude: zero exactly for +-0 +- 0i (integer units, not the FP64 pipe).
@@ -84,15 +94,31 @@ __device__ __forceinline__ unsigned nonzero_bits(double2 x) {
 	       (unsigned)__double2loint(x.y);
 }
 
+// A thread's amplitudes of a stage.
+template <typename R>
+struct Amps {
+	static constexpr unsigned kRegs = 1u << reg_bits<R>();
+	typename Vec2<R>::type v[kRegs];
+	__device__ __forceinline__ typename Vec2<R>::type &operator[](unsigned r) { return v[r]; }
+};
+
+// x + y and x - y, one packed instruction each for complex64.
+__device__ __forceinline__ float2 cadd(float2 x, float2 y) { return __fadd2_rn(x, y); }
+__device__ __forceinline__ float2 csub(float2 x, float2 y) { return __ffma2_rn(y, make_float2(-1.0f, -1.0f), x); }
+__device__ __forceinline__ double2 cadd(double2 x, double2 y) { return make_double2(radd(x.x, y.x), radd(x.y, y.y)); }
+__device__ __forceinline__ double2 csub(double2 x, double2 y) { return make_double2(rsub(x.x, y.x), rsub(x.y, y.y)); }
+
+// Zero for an amplitude that may be zero: its exponents' words are (then
+// nonzero_bits decides; sums of normal numbers never get here otherwise).
+__device__ __forceinline__ unsigned maybe_zero(double2 x) {
+	return (unsigned)(__double2hiint(x.x) | __double2hiint(x.y)) & 0x7fffffffu;
+}
+
 template <typename R, bool EXACT, unsigned I>
-__device__ __forceinline__ void op_h(typename Vec2<R>::type (&v)[kRegs], R inv) {
+__device__ __forceinline__ void op_h(Amps<R> &v, R inv) {
 	typedef typename Vec2<R>::type V;
 	auto bfly = [&](V &x, V &y) {
-		V o0, o1;
-		o0.x = radd(x.x, y.x);
-		o0.y = radd(x.y, y.y);
-		o1.x = rsub(x.x, y.x);
-		o1.y = rsub(x.y, y.y);
+		V o0 = cadd(x, y), o1 = csub(x, y);
 		if(EXACT) {
 			o0.x = rmul(o0.x, inv);
 			o0.y = rmul(o0.y, inv);
@@ -102,13 +128,14 @@ __device__ __forceinline__ void op_h(typename Vec2<R>::type (&v)[kRegs], R inv) 
 		x = o0;
 		y = o1;
 	};
+	constexpr unsigned kRegs = Amps<R>::kRegs;
 	if constexpr(EXACT) {
 		// An all-zero pair is left as it is (dense_state_backend.cpp:265).
-		bool zero = false;
+		unsigned least = ~0u;
 #pragma unroll
 		for(unsigned r = 0; r < kRegs; ++r)
-			if(!((r >> I) & 1u)) zero = zero || (nonzero_bits(v[r]) | nonzero_bits(v[r | (1u << I)])) == 0u;
-		if(__any_sync(0xffffffffu, zero)) {
+			if(!((r >> I) & 1u)) least = min(least, maybe_zero(v[r]) | maybe_zero(v[r | (1u << I)]));
+		if(least == 0u) {
 #pragma unroll
 			for(unsigned r = 0; r < kRegs; ++r)
 				if(!((r >> I) & 1u) && (nonzero_bits(v[r]) | nonzero_bits(v[r | (1u << I)])) != 0u) bfly(v[r], v[r | (1u << I)]);
@@ -122,7 +149,8 @@ __device__ __forceinline__ void op_h(typename Vec2<R>::type (&v)[kRegs], R inv) 
 
 // X on register bit I of the pairs whose register bit C is set (C == I: all).
 template <typename R, bool EXACT, unsigned I, unsigned C>
-__device__ __forceinline__ void op_x(typename Vec2<R>::type (&v)[kRegs], bool on) {
+__device__ __forceinline__ void op_x(Amps<R> &v, bool on) {
+	constexpr unsigned kRegs = Amps<R>::kRegs;
 #pragma unroll
 	for(unsigned r = 0; r < kRegs; ++r) {
 		if(((r >> I) & 1u) || (C != I && !((r >> C) & 1u))) continue;
@@ -138,17 +166,25 @@ __device__ __forceinline__ void op_x(typename Vec2<R>::type (&v)[kRegs], bool on
 
 // Phase on the registers that have all bits of M.
 template <typename R, bool EXACT, unsigned M>
-__device__ __forceinline__ void op_cp(typename Vec2<R>::type (&v)[kRegs], R pr, R pi) {
+__device__ __forceinline__ void op_cp(Amps<R> &v, R pr, R pi) {
+	constexpr unsigned kRegs = Amps<R>::kRegs;
+	unsigned least = ~0u;
+	if constexpr(EXACT) {
+#pragma unroll
+		for(unsigned r = 0; r < kRegs; ++r)
+			if((r & M) == M) least = min(least, maybe_zero(v[r]));
+	}
 #pragma unroll
 	for(unsigned r = 0; r < kRegs; ++r) {
 		if((r & M) != M) continue;
 		R re = v[r].x, im = v[r].y;
 		if constexpr(EXACT) {
 			// Zero amplitudes are skipped (dense_state_backend.cpp:299).
-			const bool nz = nonzero_bits(v[r]) != 0u;
 			cmul_ref(pr, pi, re, im);
-			v[r].x = nz ? re : v[r].x;
-			v[r].y = nz ? im : v[r].y;
+			if(least != 0u || nonzero_bits(v[r]) != 0u) {
+				v[r].x = re;
+				v[r].y = im;
+			}
 		} else {
 			v[r].x = fma(pr, re, -(pi * im));
 			v[r].y = fma(pr, im, pi * re);
@@ -156,14 +192,54 @@ __device__ __forceinline__ void op_cp(typename Vec2<R>::type (&v)[kRegs], R pr, 
 	}
 }
 
+// A matrix element g in shared memory: complex128 as it is; complex64 as the two
+// operand pairs of a packed complex product, (re, re) and (-im, im).
+template <typename R>
+struct MatElem;
+template <>
+struct MatElem<double> {
+	typedef double2 type;
+	static __device__ __forceinline__ double2 make(double2 g) { return g; }
+};
+template <>
+struct MatElem<float> {
+	typedef float4 type;
+	static __device__ __forceinline__ float4 make(double2 g) { return make_float4((float)g.x, (float)g.x, -(float)g.y, (float)g.y); }
+};
+
+// Loaded where it is used: a broadcast, and cheaper than the spills of keeping
+// the whole matrix in registers.
+__device__ __forceinline__ double2 mat_at(const double2 *m) {
+	double2 x;
+	asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.x), "=d"(x.y) : "r"((unsigned)__cvta_generic_to_shared(m)));
+	return x;
+}
+__device__ __forceinline__ float4 mat_at(const float4 *m) {
+	float4 x;
+	asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+	             : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"((unsigned)__cvta_generic_to_shared(m)));
+	return x;
+}
+
+// o += g * x in the fast forms; xs is x with its components exchanged.
+__device__ __forceinline__ void cfma(float4 g, float2 x, float2 xs, float2 &o) {
+	o = __ffma2_rn(make_float2(g.x, g.y), x, o);
+	o = __ffma2_rn(make_float2(g.z, g.w), xs, o);
+}
+__device__ __forceinline__ void cfma(double2 g, double2 x, double2, double2 &o) {
+	o.x = fma(-g.y, x.y, fma(g.x, x.x, o.x));
+	o.y = fma(g.y, x.x, fma(g.x, x.y, o.y));
+}
+
 // Dense gate on register bit I: the unrolled formula of gate_block_apply.h:117-140.
 template <typename R, bool EXACT, unsigned I>
-__device__ __forceinline__ void op_u1(typename Vec2<R>::type (&v)[kRegs], const typename Vec2<R>::type *m) {
+__device__ __forceinline__ void op_u1(Amps<R> &v, const typename MatElem<R>::type *m) {
+	typedef typename Vec2<R>::type V;
 	const auto g00 = m[0], g01 = m[1], g10 = m[2], g11 = m[3];
 #pragma unroll
-	for(unsigned r = 0; r < kRegs; ++r) {
+	for(unsigned r = 0; r < Amps<R>::kRegs; ++r) {
 		if((r >> I) & 1u) continue;
-		const auto x = v[r], y = v[r | (1u << I)];
+		const V x = v[r], y = v[r | (1u << I)];
 		if constexpr(EXACT) {
 			if((nonzero_bits(x) | nonzero_bits(y)) == 0u) continue;
 			v[r].x = rsub(radd(rsub(rmul(g00.x, x.x), rmul(g00.y, x.y)), rmul(g01.x, y.x)), rmul(g01.y, y.y));
@@ -171,109 +247,147 @@ __device__ __forceinline__ void op_u1(typename Vec2<R>::type (&v)[kRegs], const 
 			v[r | (1u << I)].x = rsub(radd(rsub(rmul(g10.x, x.x), rmul(g10.y, x.y)), rmul(g11.x, y.x)), rmul(g11.y, y.y));
 			v[r | (1u << I)].y = radd(radd(radd(rmul(g10.x, x.y), rmul(g10.y, x.x)), rmul(g11.x, y.y)), rmul(g11.y, y.x));
 		} else {
-			v[r].x = fma(-g01.y, y.y, fma(g01.x, y.x, fma(-g00.y, x.y, g00.x * x.x)));
-			v[r].y = fma(g01.y, y.x, fma(g01.x, y.y, fma(g00.y, x.x, g00.x * x.y)));
-			v[r | (1u << I)].x = fma(-g11.y, y.y, fma(g11.x, y.x, fma(-g10.y, x.y, g10.x * x.x)));
-			v[r | (1u << I)].y = fma(g11.y, y.x, fma(g11.x, y.y, fma(g10.y, x.x, g10.x * x.y)));
+			V xs, ys, o0, o1;
+			xs.x = x.y, xs.y = x.x, ys.x = y.y, ys.y = y.x;
+			o0.x = o0.y = o1.x = o1.y = R(0);
+			cfma(g00, x, xs, o0);
+			cfma(g10, x, xs, o1);
+			cfma(g01, y, ys, o0);
+			cfma(g11, y, ys, o1);
+			v[r] = o0;
+			v[r | (1u << I)] = o1;
 		}
 	}
-}
-
-// A matrix element from shared memory, loaded where it is used: a broadcast,
-// and cheaper than the spills of keeping the whole matrix in registers.
-__device__ __forceinline__ double2 mat_at(const double2 *m) {
-	double2 x;
-	asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.x), "=d"(x.y) : "r"((unsigned)__cvta_generic_to_shared(m)));
-	return x;
-}
-__device__ __forceinline__ float2 mat_at(const float2 *m) {
-	float2 x;
-	asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"((unsigned)__cvta_generic_to_shared(m)));
-	return x;
 }
 
 // Dense gate on register bits A (more significant) and B: row sums term by term
-// (gate_block_apply.h:165-176); all-zero blocks are left alone.
+// (gate_block_apply.h:165-176); all-zero blocks are left alone.  Fast forms: two
+// blocks per matrix element loaded.
 template <typename R, bool EXACT, unsigned A, unsigned B>
-__device__ __forceinline__ void op_u2(typename Vec2<R>::type (&v)[kRegs], const typename Vec2<R>::type *m) {
+__device__ __forceinline__ void op_u2(Amps<R> &v, const typename MatElem<R>::type *m) {
+	typedef typename Vec2<R>::type V;
+	constexpr unsigned RB = reg_bits<R>(), mask = (1u << A) | (1u << B);
+	// Register of index c of block b.
+	auto at = [](unsigned b, unsigned c) {
+		unsigned r = 0, k = 0;
+		for(unsigned i = 0; i < RB; ++i)
+			if(!((mask >> i) & 1u)) r |= ((b >> k++) & 1u) << i;
+		return r | ((c >> 1) << A) | ((c & 1u) << B);
+	};
+	if constexpr(EXACT) {
 #pragma unroll
-	for(unsigned r = 0; r < kRegs; ++r) {
-		if(((r >> A) & 1u) || ((r >> B) & 1u)) continue;
-		const unsigned at[4] = {r, r | (1u << B), r | (1u << A), r | (1u << A) | (1u << B)};
-		typename Vec2<R>::type o[4];
-		if constexpr(EXACT)
-			if((nonzero_bits(v[at[0]]) | nonzero_bits(v[at[1]]) | nonzero_bits(v[at[2]]) | nonzero_bits(v[at[3]])) == 0u) continue;
+		for(unsigned b = 0; b < Amps<R>::kRegs / 4; ++b) {
+			V o[4];
+			if((nonzero_bits(v[at(b, 0)]) | nonzero_bits(v[at(b, 1)]) | nonzero_bits(v[at(b, 2)]) | nonzero_bits(v[at(b, 3)])) == 0u) continue;
 #pragma unroll
-		for(unsigned row = 0; row < 4; ++row) {
-			R nr = R(0), ni = R(0);
+			for(unsigned row = 0; row < 4; ++row) {
+				V n;
+				n.x = n.y = R(0);
+#pragma unroll
+				for(unsigned c = 0; c < 4; ++c) {
+					const auto g = mat_at(m + 4 * row + c);
+					const V x = v[at(b, c)];
+					n.x = radd(n.x, rsub(rmul(g.x, x.x), rmul(g.y, x.y)));
+					n.y = radd(n.y, radd(rmul(g.x, x.y), rmul(g.y, x.x)));
+				}
+				o[row] = n;
+			}
+#pragma unroll
+			for(unsigned c = 0; c < 4; ++c) v[at(b, c)] = o[c];
+		}
+	} else {
+#pragma unroll
+		for(unsigned b = 0; b < Amps<R>::kRegs / 4; b += 2) {
+			V o[2][4];
+#pragma unroll
+			for(unsigned k = 0; k < 2; ++k)
+#pragma unroll
+				for(unsigned c = 0; c < 4; ++c) o[k][c].x = o[k][c].y = R(0);
 #pragma unroll
 			for(unsigned c = 0; c < 4; ++c) {
-				const auto g = mat_at(m + 4 * row + c), x = v[at[c]];
-				if constexpr(EXACT) {
-					nr = radd(nr, rsub(rmul(g.x, x.x), rmul(g.y, x.y)));
-					ni = radd(ni, radd(rmul(g.x, x.y), rmul(g.y, x.x)));
-				} else {
-					nr = fma(-g.y, x.y, fma(g.x, x.x, nr));
-					ni = fma(g.y, x.x, fma(g.x, x.y, ni));
+				V xs[2];
+#pragma unroll
+				for(unsigned k = 0; k < 2; ++k) {
+					xs[k].x = v[at(b + k, c)].y;
+					xs[k].y = v[at(b + k, c)].x;
+				}
+#pragma unroll
+				for(unsigned row = 0; row < 4; ++row) {
+					const auto g = mat_at(m + 4 * row + c);
+#pragma unroll
+					for(unsigned k = 0; k < 2; ++k) cfma(g, v[at(b + k, c)], xs[k], o[k][row]);
 				}
 			}
-			o[row].x = nr;
-			o[row].y = ni;
-		}
 #pragma unroll
-		for(unsigned c = 0; c < 4; ++c) v[at[c]] = o[c];
+			for(unsigned k = 0; k < 2; ++k)
+#pragma unroll
+				for(unsigned c = 0; c < 4; ++c) v[at(b + k, c)] = o[k][c];
+		}
 	}
 }
 
-template <typename R, bool EXACT>
-__device__ __forceinline__ void run_op(const GateOp &op, typename Vec2<R>::type (&v)[kRegs], const GateGeom &g, const typename Vec2<R>::type *mats, uint64_t base, unsigned t) {
-	if(op.code == kCodeFlip) {
-		const unsigned at = (base & g.outer) == op.omask && t == op.tmask ? op.rval : kRegs;
-#pragma unroll
-		for(unsigned r = 0; r < kRegs; ++r) {
-			v[r].x = r == at ? -v[r].x : v[r].x;
-			v[r].y = r == at ? -v[r].y : v[r].y;
-		}
-		return;
-	}
-	if(op.code >= kCodeU1) {
-		const typename Vec2<R>::type *m = mats + op.omask;
+template <typename R, bool EXACT, bool DENSE>
+__device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateGeom &g, const typename MatElem<R>::type *mats, uint64_t base,
+                                       unsigned t) {
+	constexpr unsigned RB = reg_bits<R>();
+	if(DENSE && op.code >= kCodeU1) {
+		const typename MatElem<R>::type *m = mats + op.omask;
 		switch(op.code) {
-#define TQB_U1(I) \
-	case kCodeU1 + I: op_u1<R, EXACT, I>(v, m); return;
-#define TQB_U2(A, B) \
-	case kCodeU2 + 4 * A + B: op_u2<R, EXACT, A, B>(v, m); return;
-			TQB_U1(0) TQB_U1(1) TQB_U1(2) TQB_U1(3)
+#define TQB_U1(I)                                                         \
+	case kCodeU1 + I:                                                     \
+		if constexpr(DENSE && I < RB) op_u1<R, EXACT, I < RB ? I : 0u>(v, m);      \
+		return;
+#define TQB_U2(A, B)                                                                                    \
+	case kCodeU2 + 5 * A + B:                                                                           \
+		if constexpr(DENSE && A < RB && B < RB && (EXACT || A > B)) op_u2<R, EXACT, A < RB ? A : 0u, B < RB ? B : 0u>(v, m); \
+		return;
+			TQB_U1(0) TQB_U1(1) TQB_U1(2) TQB_U1(3) TQB_U1(4)
 			TQB_U2(0, 1) TQB_U2(0, 2) TQB_U2(0, 3) TQB_U2(1, 0) TQB_U2(1, 2) TQB_U2(1, 3)
 			TQB_U2(2, 0) TQB_U2(2, 1) TQB_U2(2, 3) TQB_U2(3, 0) TQB_U2(3, 1) TQB_U2(3, 2)
+			TQB_U2(4, 0) TQB_U2(4, 1) TQB_U2(4, 2) TQB_U2(4, 3)
 #undef TQB_U1
 #undef TQB_U2
 			default: return;
 		}
 	}
+	if(op.code == kCodeFlip) {
+		const unsigned at = (base & g.outer) == op.omask && t == op.tmask ? op.rval : Amps<R>::kRegs;
+#pragma unroll
+		for(unsigned r = 0; r < Amps<R>::kRegs; ++r) {
+			v[r].x = r == at ? -v[r].x : v[r].x;
+			v[r].y = r == at ? -v[r].y : v[r].y;
+		}
+		return;
+	}
 	if((base & op.omask) != op.omask) return;
 	const bool on = (t & op.tmask) == op.tmask;
 	const R inv = (R)g.inv;
 	switch(op.code) {
-		case kCodeH + 0: op_h<R, EXACT, 0>(v, inv); return;
-		case kCodeH + 1: op_h<R, EXACT, 1>(v, inv); return;
-		case kCodeH + 2: op_h<R, EXACT, 2>(v, inv); return;
-		case kCodeH + 3: op_h<R, EXACT, 3>(v, inv); return;
-#define TQB_X(I, C) \
-	case kCodeX + 4 * I + C: op_x<R, EXACT, I, C>(v, on); return;
-		TQB_X(0, 0) TQB_X(0, 1) TQB_X(0, 2) TQB_X(0, 3)
-		TQB_X(1, 0) TQB_X(1, 1) TQB_X(1, 2) TQB_X(1, 3)
-		TQB_X(2, 0) TQB_X(2, 1) TQB_X(2, 2) TQB_X(2, 3)
-		TQB_X(3, 0) TQB_X(3, 1) TQB_X(3, 2) TQB_X(3, 3)
+#define TQB_H(I)                                                          \
+	case kCodeH + I:                                                      \
+		if constexpr(I < RB) op_h<R, EXACT, I < RB ? I : 0u>(v, inv);     \
+		return;
+#define TQB_XC(I, C)                                                                                       \
+	case kCodeX + 5 * I + C:                                                                               \
+		if constexpr(I < RB && C < RB) op_x<R, EXACT, I < RB ? I : 0u, C < RB ? C : 0u>(v, on);            \
+		return;
+#define TQB_X(I) TQB_XC(I, 0) TQB_XC(I, 1) TQB_XC(I, 2) TQB_XC(I, 3) TQB_XC(I, 4)
+		TQB_H(0) TQB_H(1) TQB_H(2) TQB_H(3) TQB_H(4)
+		TQB_X(0) TQB_X(1) TQB_X(2) TQB_X(3) TQB_X(4)
+#undef TQB_H
 #undef TQB_X
+#undef TQB_XC
 		default: break;
 	}
 	if(!on) return;
 	const R pr = (R)op.cr, pi = (R)op.ci;
 	switch(op.code) {
-#define TQB_CP(M) \
-	case kCodeCP + M: op_cp<R, EXACT, M>(v, pr, pi); return;
+#define TQB_CP(M)                                                                     \
+	case kCodeCP + M:                                                                 \
+		if constexpr(M < (1u << RB)) op_cp<R, EXACT, M < (1u << RB) ? M : 0u>(v, pr, pi); \
+		return;
 		TQB_CP(0) TQB_CP(1) TQB_CP(2) TQB_CP(3) TQB_CP(4) TQB_CP(5) TQB_CP(6) TQB_CP(8) TQB_CP(9) TQB_CP(10) TQB_CP(12)
+		TQB_CP(16) TQB_CP(17) TQB_CP(18) TQB_CP(20) TQB_CP(24)
 #undef TQB_CP
 		default: break;
 	}
@@ -287,22 +401,44 @@ __device__ __forceinline__ unsigned slot_of(unsigned b) {
 	return (1u << b) | (b >= s ? 1u << (b % s) : 0u);
 }
 
-template <typename R, bool EXACT>
-__global__ void __launch_bounds__(1u << (tile_bits<R>() - kRB), 2) k_gate_pass(typename Vec2<R>::type *a, const __grid_constant__ GateGeom g,
-                                                                              const GateOp *gops, const double2 *gmats) {
+// Shared memory: tile, operations, matrices, thread slots of the first stages.
+// DENSE: the pass holds dense gates (their code costs the others registers).
+template <typename R, bool EXACT, bool DENSE>
+__global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::type *a, const __grid_constant__ GateGeom g, const GateOp *gops,
+                                                           const double2 *gmats) {
 	typedef typename Vec2<R>::type V;
-	constexpr unsigned K = tile_bits<R>(), TB = K - kRB;
+	constexpr unsigned K = tile_bits<R>(), RB = reg_bits<R>(), TB = kThreadBits, kRegs = 1u << RB;
+	static_assert(RB + TB == K, "one amplitude set per thread");
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	V *s = reinterpret_cast<V *>(smem_raw);
 	GateOp *ops = reinterpret_cast<GateOp *>(smem_raw + (sizeof(V) << K));
-	V *mats = reinterpret_cast<V *>(ops + g.nops);
+	typedef typename MatElem<R>::type ME;
+	ME *mats = reinterpret_cast<ME *>(ops + g.nops);
+	uint16_t *slots = reinterpret_cast<uint16_t *>(mats + g.nmat);
 	const unsigned t = threadIdx.x;
 	for(unsigned e = t; e < g.nops * (sizeof(GateOp) / 16); e += blockDim.x)
 		reinterpret_cast<int4 *>(ops)[e] = reinterpret_cast<const int4 *>(gops)[e];
-	for(unsigned e = t; e < g.nmat; e += blockDim.x) {
-		const double2 x = gmats[e];
-		mats[e].x = (R)x.x;
-		mats[e].y = (R)x.y;
+	for(unsigned e = t; e < g.nmat; e += blockDim.x) mats[e] = MatElem<R>::make(gmats[e]);
+	// Where this thread's amplitudes sit in shared memory in a stage (register 0).
+	auto thread_slot = [&](unsigned st) {
+		unsigned x = 0;
+#pragma unroll
+		for(unsigned k = 0; k < TB; ++k) x ^= (t >> k) & 1u ? slot_of<R>(g.tbit[st][k]) : 0u;
+		return x;
+	};
+	for(unsigned st = 0; st < min(g.nstages, kSlotStages); ++st) slots[st * kThreads + t] = (uint16_t)thread_slot(st);
+	// And in HBM, when the tile is loaded and stored.
+	V *pin = a, *pout = a;
+	{
+		const unsigned e = g.nstages - 1u;
+		uint64_t x = 0, y = 0;
+#pragma unroll
+		for(unsigned k = 0; k < TB; ++k) {
+			x |= (uint64_t)((t >> k) & 1u) << g.lpos[g.tbit[0][k]];
+			y |= (uint64_t)((t >> k) & 1u) << g.opos[g.tbit[e][k]];
+		}
+		pin += x;
+		pout += y;
 	}
 	__syncthreads();
 	for(uint64_t o = g.o_begin + blockIdx.x; o < g.ntiles; o += gridDim.x) {
@@ -311,60 +447,43 @@ __global__ void __launch_bounds__(1u << (tile_bits<R>() - kRB), 2) k_gate_pass(t
 		for(unsigned i = 0; i < K; ++i) base = insert0(base, g.lpos[i]);
 		for(unsigned st = 0; st < g.nstages; ++st) {
 			const bool last = st + 1 == g.nstages;
-			V v[kRegs];
-			// Where this thread's amplitudes sit in shared memory.
-			unsigned slot = 0, ro[kRB];
+			Amps<R> v;
+			const unsigned slot = st < kSlotStages ? slots[st * kThreads + t] : thread_slot(st);
+			unsigned ro[RB];
 #pragma unroll
-			for(unsigned k = 0; k < TB; ++k) slot ^= (t >> k) & 1u ? slot_of<R>(g.tbit[st][k]) : 0u;
-#pragma unroll
-			for(unsigned i = 0; i < kRB; ++i) ro[i] = slot_of<R>(g.rbit[st][i]);
+			for(unsigned i = 0; i < RB; ++i) ro[i] = slot_of<R>(g.rbit[st][i]);
 			auto at = [&](unsigned r) {
-				unsigned x = slot;
+				unsigned x = 0;
 #pragma unroll
-				for(unsigned i = 0; i < kRB; ++i)
+				for(unsigned i = 0; i < RB; ++i)
 					if((r >> i) & 1u) x ^= ro[i];
-				return x;
+				return slot ^ x;
 			};
-			// And in HBM.
-			auto global = [&](const uint8_t *pos, uint64_t (&go)[kRB]) {
+			// Offset of register r from the thread's place in HBM (uniform).
+			auto global = [&](const uint8_t *pos, unsigned r) {
 				uint64_t x = base;
 #pragma unroll
-				for(unsigned k = 0; k < TB; ++k) x |= (uint64_t)((t >> k) & 1u) << pos[g.tbit[st][k]];
-#pragma unroll
-				for(unsigned i = 0; i < kRB; ++i) go[i] = 1ull << pos[g.rbit[st][i]];
+				for(unsigned i = 0; i < RB; ++i)
+					if((r >> i) & 1u) x |= 1ull << pos[g.rbit[st][i]];
 				return x;
 			};
 			if(st == 0) {
-				uint64_t go[kRB];
-				const uint64_t gb = global(g.lpos, go);
 #pragma unroll
-				for(unsigned r = 0; r < kRegs; ++r) {
-					uint64_t x = gb;
-#pragma unroll
-					for(unsigned i = 0; i < kRB; ++i)
-						if((r >> i) & 1u) x |= go[i];
-					v[r] = a[x];
-				}
+				for(unsigned r = 0; r < kRegs; ++r) v[r] = pin[global(g.lpos, r)];
 			} else {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) v[r] = s[at(r)];
 			}
 			const unsigned k1 = (unsigned)g.first[st] + g.count[st];
-			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT>(ops[k], v, g, mats, base, t);
+			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT, DENSE>(ops[k], v, g, mats, base, t);
 			if(last) {
-				uint64_t go[kRB];
-				const uint64_t gb = global(g.opos, go);
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) {
-					uint64_t x = gb;
-#pragma unroll
-					for(unsigned i = 0; i < kRB; ++i)
-						if((r >> i) & 1u) x |= go[i];
 					if(!EXACT) {
 						v[r].x *= (R)g.scale;
 						v[r].y *= (R)g.scale;
 					}
-					a[x] = v[r];
+					pout[global(g.opos, r)] = v[r];
 				}
 			} else {
 #pragma unroll
@@ -388,7 +507,8 @@ struct PlanOp {
 };
 
 // The stage plan of a pass; false: it does not fit (another kernel runs it).
-bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, std::vector<GateOp> &out) {
+bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, bool exact, GateGeom &g, std::vector<GateOp> &out,
+                std::vector<double> &mats) {
 	if(pass.K != K || pass.ops.empty() || pass.n < K) return false;
 	g = GateGeom{};
 	g.n = pass.n;
@@ -478,7 +598,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 		if(g.lpos[b] < low) keep_in |= 1u << b;
 		if(g.opos[b] < low) keep_out |= 1u << b;
 	}
-	// Stages: consecutive operations while their targets fit in four register bits.
+	// Stages: consecutive operations while their targets fit in the register bits.
 	std::vector<uint32_t> regs{0u};
 	std::vector<std::vector<unsigned>> of(1);
 	for(unsigned k = 0; k < ops.size(); ++k) {
@@ -486,7 +606,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 		if(ops[k].kind != PlanOp::kCP && ops[k].kind != PlanOp::kFlip) bits = 1u << ops[k].p;
 		if(ops[k].kind == PlanOp::kU2) bits |= 1u << ops[k].p2;
 		if(bits & ~regs.back()) {
-			if(__builtin_popcount(regs.back() | bits) > (int)kRB || (regs.size() == 1 && (keep_in & bits))) {
+			if(__builtin_popcount(regs.back() | bits) > (int)RB || (regs.size() == 1 && (keep_in & bits))) {
 				regs.push_back(bits);
 				of.push_back({});
 			} else {
@@ -505,6 +625,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 	g.nstages = (unsigned)regs.size();
 	if(g.nstages > kMaxStages) return false;
 	out.clear();
+	mats = pass.mats;
 	for(unsigned st = 0; st < g.nstages; ++st) {
 		const bool in = st == 0, outs = st + 1 == g.nstages;
 		const uint32_t fixed = (in ? keep_in : 0u) | (outs ? keep_out : 0u);
@@ -515,7 +636,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 		for(unsigned k : of[st])
 			for(unsigned b = 0; b < K; ++b) cost[b] += ops[k].kind != PlanOp::kFlip && ((ops[k].pm >> b) & 1u);
 		uint32_t r = regs[st];
-		while(__builtin_popcount(r) < (int)kRB) {
+		while(__builtin_popcount(r) < (int)RB) {
 			int best = -1;
 			for(int b = (int)K - 1; b >= 0; --b)
 				if(!((r | fixed) >> b & 1u) && (best < 0 || cost[b] > cost[best])) best = b;
@@ -546,7 +667,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 					}
 		}
 		while(!rest.empty()) take(rest.front());
-		for(unsigned i = 0; i < kRB; ++i) g.rbit[st][i] = (uint8_t)rb[i];
+		for(unsigned i = 0; i < RB; ++i) g.rbit[st][i] = (uint8_t)rb[i];
 		for(unsigned k = 0; k < tb.size(); ++k) g.tbit[st][k] = (uint8_t)tb[k];
 		g.first[st] = (uint8_t)out.size();
 		g.count[st] = (uint8_t)of[st].size();
@@ -554,10 +675,10 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 			const PlanOp &q = ops[k];
 			GateOp o{};
 			uint32_t rm = 0, tm = 0;
-			for(unsigned i = 0; i < kRB; ++i) rm |= ((q.pm >> rb[i]) & 1u) << i;
+			for(unsigned i = 0; i < RB; ++i) rm |= ((q.pm >> rb[i]) & 1u) << i;
 			for(unsigned i = 0; i < tb.size(); ++i) tm |= ((q.pm >> tb[i]) & 1u) << i;
 			unsigned target = 0, second = 0;
-			for(unsigned i = 0; i < kRB; ++i) {
+			for(unsigned i = 0; i < RB; ++i) {
 				if(rb[i] == q.p) target = i;
 				if(rb[i] == q.p2) second = i;
 			}
@@ -567,7 +688,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 			o.ci = q.ci;
 			switch(q.kind) {
 				case PlanOp::kH: o.code = kCodeH + target; break;
-				case PlanOp::kX: o.code = kCodeX + 4 * target + (rm ? (unsigned)__builtin_ctz(rm) : target); break;
+				case PlanOp::kX: o.code = kCodeX + 5 * target + (rm ? (unsigned)__builtin_ctz(rm) : target); break;
 				case PlanOp::kCP: o.code = kCodeCP + rm; break;
 				case PlanOp::kFlip:
 					o.code = kCodeFlip;
@@ -575,7 +696,19 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 					break;
 				case PlanOp::kU1:
 				case PlanOp::kU2:
-					o.code = q.kind == PlanOp::kU1 ? kCodeU1 + target : kCodeU2 + 4 * target + second;
+					if(q.kind == PlanOp::kU2 && !exact && target < second) {
+						// The block index with its two bits exchanged (exact: the order of
+						// the row sums is the gate's own).
+						std::swap(target, second);
+						double *m = mats.data() + 2 * q.mat;
+						const unsigned x[4] = {0, 2, 1, 3};
+						double y[32];
+						for(unsigned r = 0; r < 4; ++r)
+							for(unsigned c = 0; c < 4; ++c)
+								for(unsigned k2 = 0; k2 < 2; ++k2) y[2 * (4 * x[r] + x[c]) + k2] = m[2 * (4 * r + c) + k2];
+						std::copy(y, y + 32, m);
+					}
+					o.code = q.kind == PlanOp::kU1 ? kCodeU1 + target : kCodeU2 + 5 * target + second;
 					o.omask = q.mat;
 					break;
 			}
@@ -584,7 +717,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned line, GateGeom &g, s
 	}
 	g.nops = (unsigned)out.size();
 	g.nmat = (unsigned)(pass.mats.size() / 2);
-	g.scale = std::pow(2.0, -0.5 * (double)nh);
+	g.scale = std::pow(g.inv, (double)nh);  // of the reference's 1/sqrt(2), rounded as it is: the difference adds up
 	return true;
 }
 
@@ -593,8 +726,9 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	constexpr unsigned K = tile_bits<R>();
 	GateGeom g;
 	std::vector<GateOp> ops;
-	if(!plan_gates(pass, K, line_bits<R>(), g, ops)) return false;
-	const size_t ops_bytes = ops.size() * sizeof(GateOp), mat_bytes = pass.mats.size() * sizeof(double);
+	std::vector<double> mats;
+	if(!plan_gates(pass, K, reg_bits<R>(), line_bits<R>(), EXACT, g, ops, mats)) return false;
+	const size_t ops_bytes = ops.size() * sizeof(GateOp), mat_bytes = mats.size() * sizeof(double);
 	const size_t need = std::max<size_t>(sizeof(GateOp), ops_bytes + mat_bytes);
 	if(need > dev_prog_bytes) {
 		if(dev_prog) {
@@ -611,17 +745,16 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	}
 	std::vector<unsigned char> host(need);
 	if(ops_bytes) std::memcpy(host.data(), ops.data(), ops_bytes);
-	if(mat_bytes) std::memcpy(host.data() + ops_bytes, pass.mats.data(), mat_bytes);
+	if(mat_bytes) std::memcpy(host.data() + ops_bytes, mats.data(), mat_bytes);
 	if(ops_bytes + mat_bytes) upload_async(c, dev_prog, host.data(), ops_bytes + mat_bytes, "gate pass program upload");
 	typedef typename Vec2<R>::type V;
-	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(V);
-	auto kern = k_gate_pass<R, EXACT>;
+	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(typename MatElem<R>::type) + sizeof(uint16_t) * kThreads * std::min(g.nstages, kSlotStages);
+	auto kern = mats.empty() ? k_gate_pass<R, EXACT, false> : k_gate_pass<R, EXACT, true>;
 	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gate pass smem");
-	const unsigned threads = 1u << (K - kRB);
 	int per_sm = 1;
-	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem), "gate pass occupancy");
+	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem), "gate pass occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));
-	kern<<<(unsigned)grid, threads, smem, c.stream>>>(static_cast<V *>(a), g, static_cast<const GateOp *>(dev_prog),
+	kern<<<(unsigned)grid, kThreads, smem, c.stream>>>(static_cast<V *>(a), g, static_cast<const GateOp *>(dev_prog),
 	                                                 reinterpret_cast<const double2 *>(static_cast<unsigned char *>(dev_prog) + ops_bytes));
 	check_cuda(cudaGetLastError(), "gate pass");
 	if(c.launches) ++*c.launches;
