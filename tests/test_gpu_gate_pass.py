@@ -107,6 +107,34 @@ def test_more_operations_than_one_plan_holds(prec):
         assert O.rel_l2(ref, got) <= 400 * 2.0 ** -24
 
 
+def rings(n, layers, seed, extra):
+    """Hadamard layers with rings of phases, and `extra` random phases after each (pairs in every position)."""
+    rng = np.random.default_rng(seed)
+    ops = []
+    for _ in range(layers):
+        ops += [lambda M, q=q: M.h(q) for q in range(n)]
+        pairs = [(q, (q + 1) % n) for q in range(n)] + [tuple(int(v) for v in rng.permutation(n)[:2]) for _ in range(extra)]
+        ops += [lambda M, c=c, q=q, x=float(rng.uniform(-4, 4)): M.cphase(c, q, x) for c, q in pairs]
+    return ops
+
+
+@pytest.mark.parametrize("n", [12, 13, 14, 15, 17, 19])
+@pytest.mark.parametrize("form", ["c64", "f64fast"])
+@pytest.mark.parametrize("extra", [0, 40])
+def test_merged_phase_runs(n, form, extra):
+    ops = rings(n, 3, n, extra)
+    a = inputs("random", n, n)
+    r = O.OracleRegister(n, amps=a)
+    r.run([f(O) for f in ops])
+    with tq.GpuState(tq.FP32 if form == "c64" else tq.FP64) as g:
+        if form == "f64fast":
+            g.set_option(tq.OPT_EXACT, 0)
+        g.load(n, a)
+        g.apply_ops([f(tq) for f in ops])
+        got = g.export()
+    assert O.rel_l2(r.amplitudes(), got) <= len(ops) * (2.0 ** -24 if form == "c64" else 2.0 ** -53)
+
+
 @pytest.mark.parametrize("n", [20, 22])
 def test_relabelled_tiles_of_one_stage(n):
     """A swap and few targets: one register stage, several tiles per block, every amplitude stored elsewhere in its tile."""

@@ -144,13 +144,12 @@ __device__ __forceinline__ V cmul(V a, V b) {
 template <typename R, typename A>
 __global__ void __launch_bounds__(kAdjThreads, 2) k_grad_run(typename Vec2<R>::type *lam, typename Vec2<R>::type *psi,
                                                             uint64_t N, RunParams rp, unsigned nbytes, int uncompute_psi,
-                                                            double *partials) {
+                                                            unsigned shares, double *partials) {
 	typedef typename Vec2<R>::type V;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	A *accs = reinterpret_cast<A *>(smem_raw);                                              // [warps][entries][32]
 	V *qtab = reinterpret_cast<V *>(accs + (kAdjThreads / 32) * kMaxDiagRun * 32);           // [4][256]
 	uint32_t *tab = reinterpret_cast<uint32_t *>(qtab + 4 * 256);                           // [nbytes][256]
-	__shared__ double red[kAdjThreads / 32];
 	__shared__ uint32_t cls[kGradBatch];
 	const unsigned count = rp.count;
 	const unsigned nq = (count + 7) / 8;  // phase tables in use
@@ -191,8 +190,6 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_grad_run(typename Vec2<R>::t
 		}
 		tab[j ? e : (((v & 7u) << 5) | (v >> 3))] = bits;
 	}
-	for(unsigned e = threadIdx.x; e < (kAdjThreads / 32) * kMaxDiagRun * 32; e += blockDim.x) accs[e] = A(0);
-	__syncthreads();
 	const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	A *col = accs + warp * kMaxDiagRun * 32 + lane;
 	const uint32_t all = count >= 32 ? ~0u : ((1u << count) - 1u);
@@ -205,122 +202,131 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_grad_run(typename Vec2<R>::t
 	// The entries that depend on the three lowest index bits come first and
 	// number at most 8: bytes 1-3 of the hit word are the same for the batch.
 	const bool split = nq > 1 && rp.nvary <= 8;
-	for(uint64_t x0 = gtid() * kGradBatch; x0 < N; x0 += gstride() * kGradBatch) {
-		V lb[kGradBatch], pb[kGradBatch];
-		if constexpr(sizeof(V) == 8) {
-			if(lim == kGradBatch) {
-				// Eight complex64 values: two 32-byte loads each (x0 is a multiple of 8).
+	// The work is cut into `shares` strided shares, each with its own columns and
+	// its own row of partial sums; a block takes one after the other.
+	for(unsigned share = blockIdx.x; share < shares; share += gridDim.x) {
+		__syncthreads();
+		for(unsigned e = threadIdx.x; e < (kAdjThreads / 32) * kMaxDiagRun * 32; e += blockDim.x) accs[e] = A(0);
+		__syncthreads();
+		for(uint64_t x0 = ((uint64_t)share * kAdjThreads + threadIdx.x) * kGradBatch; x0 < N;
+		    x0 += (uint64_t)shares * kAdjThreads * kGradBatch) {
+			V lb[kGradBatch], pb[kGradBatch];
+			if constexpr(sizeof(V) == 8) {
+				if(lim == kGradBatch) {
+					// Eight complex64 values: two 32-byte loads each (x0 is a multiple of 8).
 #pragma unroll
-				for(unsigned q = 0; q < kGradBatch / 4; ++q) {
-					float a[8], b[8];
-					ld_global_v8f(reinterpret_cast<const float *>(lam + x0 + 4 * q), a);
-					ld_global_v8f(reinterpret_cast<const float *>(psi + x0 + 4 * q), b);
+					for(unsigned q = 0; q < kGradBatch / 4; ++q) {
+						float a[8], b[8];
+						ld_global_v8f(reinterpret_cast<const float *>(lam + x0 + 4 * q), a);
+						ld_global_v8f(reinterpret_cast<const float *>(psi + x0 + 4 * q), b);
 #pragma unroll
-					for(unsigned u = 0; u < 4; ++u) {
-						lb[4 * q + u] = V{a[2 * u], a[2 * u + 1]};
-						pb[4 * q + u] = V{b[2 * u], b[2 * u + 1]};
+						for(unsigned u = 0; u < 4; ++u) {
+							lb[4 * q + u] = V{a[2 * u], a[2 * u + 1]};
+							pb[4 * q + u] = V{b[2 * u], b[2 * u + 1]};
+						}
 					}
 				}
 			}
-		}
-#pragma unroll
-		for(unsigned u = 0; u < kGradBatch; ++u)
-			if(u < lim && (sizeof(V) != 8 || lim < kGradBatch)) {
-				lb[u] = lam[x0 + u];
-				pb[u] = psi[x0 + u];
-			}
-		uint32_t hh = all;
-		for(unsigned j = 1; j < nbytes; ++j) hh &= tab[(j << 8) | ((unsigned)(x0 >> (8 * j)) & 255u)];
-		const unsigned b0s = ((unsigned)x0 & 255u) >> 3;  // byte 0 of x0, transposed index
-		// Entries 8 and up hit all eight amplitudes alike (split runs): their
-		// phase product once per batch.
-		V Prest;
-		if(split) {
-			const uint32_t h7 = hh & tab[((kGradBatch - 1) << 5) | b0s];
-			Prest = qtab[256 | ((h7 >> 8) & 255u)];
-			if(nq > 2) Prest = cmul<V, R>(Prest, qtab[512 | ((h7 >> 16) & 255u)]);
-			if(nq > 3) Prest = cmul<V, R>(Prest, qtab[768 | (h7 >> 24)]);
-		}
-		A S[kGradBatch];
-		// complex64: the results wait in registers for 16-byte stores.
-		V lo[sizeof(V) == 8 ? kGradBatch : 1], po[sizeof(V) == 8 ? kGradBatch : 1];
-#pragma unroll
-		for(unsigned u = 0; u < kGradBatch; ++u) {
-			S[u] = A(0);
-			if(u >= lim) continue;
-			V l = lb[u], p = pb[u];
-			S[u] = (A)l.y * (A)p.x - (A)l.x * (A)p.y;
-			// Table entry 0 is the empty product 1, which leaves a value unchanged.
-			const uint32_t hit = hh & tab[(u << 5) | b0s];
-			V P = qtab[hit & 255u];
-			if(split) {
-				P = cmul<V, R>(P, Prest);
-			} else {
-				if(nq > 1) P = cmul<V, R>(P, qtab[256 | ((hit >> 8) & 255u)]);
-				if(nq > 2) P = cmul<V, R>(P, qtab[512 | ((hit >> 16) & 255u)]);
-				if(nq > 3) P = cmul<V, R>(P, qtab[768 | (hit >> 24)]);
-			}
-			if(sizeof(V) == 8 && lim == kGradBatch) {
-				lo[sizeof(V) == 8 ? u : 0] = cmul<V, R>(l, P);
-				po[sizeof(V) == 8 ? u : 0] = cmul<V, R>(p, P);
-			} else {
-				lam[x0 + u] = cmul<V, R>(l, P);
-				if(uncompute_psi) psi[x0 + u] = cmul<V, R>(p, P);
-			}
-		}
-		if constexpr(sizeof(V) == 8) {
-			if(lim == kGradBatch) {
-#pragma unroll
-				for(unsigned q = 0; q < kGradBatch / 4; ++q) {
-					float a[8], b[8];
-#pragma unroll
-					for(unsigned u = 0; u < 4; ++u) {
-						a[2 * u] = lo[4 * q + u].x;
-						a[2 * u + 1] = lo[4 * q + u].y;
-						b[2 * u] = po[4 * q + u].x;
-						b[2 * u + 1] = po[4 * q + u].y;
-					}
-					st_global_v8f(reinterpret_cast<float *>(lam + x0 + 4 * q), a);
-					if(uncompute_psi) st_global_v8f(reinterpret_cast<float *>(psi + x0 + 4 * q), b);
-				}
-			}
-		}
-		// Superset sums over the three low bits.
-#pragma unroll
-		for(unsigned b = 0; b < 3; ++b)
 #pragma unroll
 			for(unsigned u = 0; u < kGradBatch; ++u)
-				if(!((u >> b) & 1u)) S[u] += S[u | (1u << b)];
-		const uint32_t rest = hh & tab[((kGradBatch - 1) << 5) | b0s] & ~flips;
-		if(rest) {
-			// Columns of distinct entries never alias: the next column is read
-			// before the current one is written, so the reads overlap.
-#pragma unroll
-			for(unsigned c = 0; c < kGradBatch; ++c) {
-				uint32_t m = rest & cm[c];
-				if(!m) continue;
-				A *p = col + (__ffs(m) - 1) * 32;
-				A cur = *p;
-				for(m &= m - 1u; m; m &= m - 1u) {
-					A *q = col + (__ffs(m) - 1) * 32;
-					const A nxt = *q;
-					*p = cur + S[c];
-					p = q;
-					cur = nxt;
+				if(u < lim && (sizeof(V) != 8 || lim < kGradBatch)) {
+					lb[u] = lam[x0 + u];
+					pb[u] = psi[x0 + u];
 				}
-				*p = cur + S[c];
+			uint32_t hh = all;
+			for(unsigned j = 1; j < nbytes; ++j) hh &= tab[(j << 8) | ((unsigned)(x0 >> (8 * j)) & 255u)];
+			const unsigned b0s = ((unsigned)x0 & 255u) >> 3;  // byte 0 of x0, transposed index
+			// Entries 8 and up hit all eight amplitudes alike (split runs): their
+			// phase product once per batch.
+			V Prest;
+			if(split) {
+				const uint32_t h7 = hh & tab[((kGradBatch - 1) << 5) | b0s];
+				Prest = qtab[256 | ((h7 >> 8) & 255u)];
+				if(nq > 2) Prest = cmul<V, R>(Prest, qtab[512 | ((h7 >> 16) & 255u)]);
+				if(nq > 3) Prest = cmul<V, R>(Prest, qtab[768 | (h7 >> 24)]);
+			}
+			A S[kGradBatch];
+			// complex64: the results wait in registers for 16-byte stores.
+			V lo[sizeof(V) == 8 ? kGradBatch : 1], po[sizeof(V) == 8 ? kGradBatch : 1];
+#pragma unroll
+			for(unsigned u = 0; u < kGradBatch; ++u) {
+				S[u] = A(0);
+				if(u >= lim) continue;
+				V l = lb[u], p = pb[u];
+				S[u] = (A)l.y * (A)p.x - (A)l.x * (A)p.y;
+				// Table entry 0 is the empty product 1, which leaves a value unchanged.
+				const uint32_t hit = hh & tab[(u << 5) | b0s];
+				V P = qtab[hit & 255u];
+				if(split) {
+					P = cmul<V, R>(P, Prest);
+				} else {
+					if(nq > 1) P = cmul<V, R>(P, qtab[256 | ((hit >> 8) & 255u)]);
+					if(nq > 2) P = cmul<V, R>(P, qtab[512 | ((hit >> 16) & 255u)]);
+					if(nq > 3) P = cmul<V, R>(P, qtab[768 | (hit >> 24)]);
+				}
+				if(sizeof(V) == 8 && lim == kGradBatch) {
+					lo[sizeof(V) == 8 ? u : 0] = cmul<V, R>(l, P);
+					po[sizeof(V) == 8 ? u : 0] = cmul<V, R>(p, P);
+				} else {
+					lam[x0 + u] = cmul<V, R>(l, P);
+					if(uncompute_psi) psi[x0 + u] = cmul<V, R>(p, P);
+				}
+			}
+			if constexpr(sizeof(V) == 8) {
+				if(lim == kGradBatch) {
+#pragma unroll
+					for(unsigned q = 0; q < kGradBatch / 4; ++q) {
+						float a[8], b[8];
+#pragma unroll
+						for(unsigned u = 0; u < 4; ++u) {
+							a[2 * u] = lo[4 * q + u].x;
+							a[2 * u + 1] = lo[4 * q + u].y;
+							b[2 * u] = po[4 * q + u].x;
+							b[2 * u + 1] = po[4 * q + u].y;
+						}
+						st_global_v8f(reinterpret_cast<float *>(lam + x0 + 4 * q), a);
+						if(uncompute_psi) st_global_v8f(reinterpret_cast<float *>(psi + x0 + 4 * q), b);
+					}
+				}
+			}
+			// Superset sums over the three low bits.
+#pragma unroll
+			for(unsigned b = 0; b < 3; ++b)
+#pragma unroll
+				for(unsigned u = 0; u < kGradBatch; ++u)
+					if(!((u >> b) & 1u)) S[u] += S[u | (1u << b)];
+			const uint32_t rest = hh & tab[((kGradBatch - 1) << 5) | b0s] & ~flips;
+			if(rest) {
+				// Columns of distinct entries never alias: the next column is read
+				// before the current one is written, so the reads overlap.
+#pragma unroll
+				for(unsigned c = 0; c < kGradBatch; ++c) {
+					uint32_t m = rest & cm[c];
+					if(!m) continue;
+					A *p = col + (__ffs(m) - 1) * 32;
+					A cur = *p;
+					for(m &= m - 1u; m; m &= m - 1u) {
+						A *q = col + (__ffs(m) - 1) * 32;
+						const A nxt = *q;
+						*p = cur + S[c];
+						p = q;
+						cur = nxt;
+					}
+					*p = cur + S[c];
+				}
 			}
 		}
-	}
-	__syncthreads();
-	// Entry k: sum its column of every warp (fixed order), then the block.
-	for(unsigned k = 0; k < count; ++k) {
-		double t = 0.0;
-		const A *ck = accs + k * 32 + lane;
-		for(unsigned w = 0; w < kAdjThreads / 32; ++w) t += (double)ck[w * kMaxDiagRun * 32];
-		// Each warp holds the same t per lane; block_sum adds the lanes of every warp.
-		const double s = block_sum(warp == 0 ? t : 0.0, red);
-		if(threadIdx.x == 0) partials[blockIdx.x * kMaxDiagRun + k] = s;
+		__syncthreads();
+		// Entry k: its columns of every warp added lane by lane in warp order, then the
+		// lanes (one warp per entry).
+		for(unsigned k = warp; k < count; k += kAdjThreads / 32) {
+			double t = 0.0;
+			const A *ck = accs + k * 32 + lane;
+			for(unsigned w = 0; w < kAdjThreads / 32; ++w) t += (double)ck[w * kMaxDiagRun * 32];
+#pragma unroll
+			for(int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+			if(lane == 0) partials[share * kMaxDiagRun + k] = t;
+		}
 	}
 }
 
@@ -409,23 +415,26 @@ unsigned launch_grad_run(const LaunchCtx &c, int prec, void *lam, void *psi, uns
 	for(unsigned k = rp.nvary; k < count; ++k)
 		if(entries[k].kind == kDiagFlip || (entries[k].mask & 7u)) rp.nvary = count;  // not ordered: no split
 	const uint64_t N = 1ull << n;
-	const unsigned blocks = adj_blocks(c, N);
+	// As many blocks as are resident (two per SM; 85 registers for three spill):
+	// each sets up its tables once.  24 phases on 2^24 complex64 amplitudes: 98 us,
+	// 119 with a block per share and a block-wide sum per entry (62 us for the bytes).
+	const unsigned shares = adj_blocks(c, N), blocks = std::min(shares, (unsigned)c.num_sms * 2u);
 	const int up = uncompute_psi ? 1 : 0;
 	const unsigned nbytes = (n + 7) / 8;
 	if(prec == TMFQS_FP64) {
 		const size_t smem = grad_smem(sizeof(double), sizeof(double2), nbytes);
 		check_cuda(cudaFuncSetAttribute(k_grad_run<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gradient smem");
 		k_grad_run<double, double><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<double2 *>(lam), static_cast<double2 *>(psi), N, rp,
-		                                                                    nbytes, up, dev_partials);
+		                                                                    nbytes, up, shares, dev_partials);
 	} else {
 		const size_t smem = grad_smem(sizeof(float), sizeof(float2), nbytes);
 		check_cuda(cudaFuncSetAttribute(k_grad_run<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gradient smem");
 		k_grad_run<float, float><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<float2 *>(lam), static_cast<float2 *>(psi), N, rp,
-		                                                                  nbytes, up, dev_partials);
+		                                                                  nbytes, up, shares, dev_partials);
 	}
 	check_cuda(cudaGetLastError(), "gradient run");
 	if(c.launches) ++*c.launches;
-	return blocks;
+	return shares;
 }
 
 }  // namespace tqb

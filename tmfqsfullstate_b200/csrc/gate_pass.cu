@@ -68,7 +68,18 @@ constexpr unsigned line_bits() {
 // set; kCodeFlip; kCodeU1 + register bit; kCodeU2 + 5 * first + second register
 // bit (the first is the more significant one of the gate's block index; in the
 // fast forms always the higher one).
-constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeFlip = 62, kCodeU1 = 63, kCodeU2 = 68;
+// kCodeDiag: a merged run of controlled phases, tmask the register bits with a
+// factor, rval its number, omask the thread bits with a factor per tile.
+constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeFlip = 62, kCodeU1 = 63, kCodeU2 = 68, kCodeDiag = 100;
+
+// Merged runs of controlled phases (fast complex128 form).  In a run the phases commute, so
+// those without two register bits collect into one factor per thread and one
+// per register bit: a part that depends on the thread index only, formed once
+// per launch (entry 0: all amplitudes, 1 + i: those with register bit i), and
+// one that depends on the tile, formed once per tile (the same entries, then
+// 6 + k: for threads with thread bit k).  Both are products in FP64, rounded once.
+constexpr unsigned kMaxLoose = 8;
+constexpr unsigned kMaxDiag = 2, kDiagMin = 6, kDiagThread = 6, kDiagTile = 6 + 8;
 
 struct GateOp {
 	uint32_t code;
@@ -79,6 +90,8 @@ struct GateOp {
 
 struct GateGeom {
 	unsigned n, nstages, nops, nmat;  // nmat: complex matrix elements of the dense gates
+	unsigned ndiag, nterms;           // merged phase runs, and the phases in them (after the operations)
+	uint16_t term[kMaxDiag][kDiagThread + kDiagTile + 1];  // first phase of each entry: the thread's, then the tile's
 	uint64_t o_begin, ntiles;  // the launch runs tiles [o_begin, ntiles)
 	double inv, scale;  // 1/sqrt(2); fast forms: the pass's power of it
 	uint64_t outer;     // mask of the index bits outside the tile
@@ -326,10 +339,45 @@ __device__ __forceinline__ void op_u2(Amps<R> &v, const typename MatElem<R>::typ
 	}
 }
 
-template <typename R, bool EXACT, bool DENSE>
-__device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateGeom &g, const typename MatElem<R>::type *mats, uint64_t base,
-                                       unsigned t) {
+template <typename V>
+__device__ __forceinline__ V cprod(V a, V b) {
+	V o;
+	o.x = fma(a.x, b.x, -(a.y * b.y));
+	o.y = fma(a.x, b.y, a.y * b.x);
+	return o;
+}
+
+// A merged run: dth this run's thread entries (per thread), dti its tile entries.
+template <typename R>
+__device__ __forceinline__ void op_diag(const GateOp &op, Amps<R> &v, const typename Vec2<R>::type *dth, const typename Vec2<R>::type *dti,
+                                        unsigned t) {
+	typedef typename Vec2<R>::type V;
+	constexpr unsigned RB = reg_bits<R>(), kRegs = Amps<R>::kRegs;
+	V p = cprod(dth[t], dti[0]);
+	for(unsigned m = (unsigned)op.omask; m; m &= m - 1u) {
+		const unsigned k = __ffs(m) - 1;
+		if((t >> k) & 1u) p = cprod(p, dti[6 + k]);
+	}
+#pragma unroll
+	for(unsigned r = 0; r < kRegs; ++r) v[r] = cprod(p, v[r]);
+#pragma unroll
+	for(unsigned i = 0; i < RB; ++i) {
+		if(!((op.tmask >> i) & 1u)) continue;
+		const V f = cprod(dth[(1 + i) * kThreads + t], dti[1 + i]);
+#pragma unroll
+		for(unsigned r = 0; r < kRegs; ++r)
+			if((r >> i) & 1u) v[r] = cprod(f, v[r]);
+	}
+}
+
+template <typename R, bool EXACT, bool DENSE, bool MERGED>
+__device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateGeom &g, const typename MatElem<R>::type *mats,
+                                       const typename Vec2<R>::type *dth, const typename Vec2<R>::type *dti, uint64_t base, unsigned t) {
 	constexpr unsigned RB = reg_bits<R>();
+	if(MERGED && op.code == kCodeDiag) {
+		op_diag<R>(op, v, dth + op.rval * kDiagThread * kThreads, dti + op.rval * kDiagTile, t);
+		return;
+	}
 	if(DENSE && op.code >= kCodeU1) {
 		const typename MatElem<R>::type *m = mats + op.omask;
 		switch(op.code) {
@@ -401,22 +449,29 @@ __device__ __forceinline__ unsigned slot_of(unsigned b) {
 	return (1u << b) | (b >= s ? 1u << (b % s) : 0u);
 }
 
-// Shared memory: tile, operations, matrices, thread slots of the first stages.
-// DENSE: the pass holds dense gates (their code costs the others registers).
-template <typename R, bool EXACT, bool DENSE>
-__global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::type *a, const __grid_constant__ GateGeom g, const GateOp *gops,
-                                                           const double2 *gmats) {
+// What a pass holds beside the plain operations: each costs the others registers.
+enum Extra { kPlain, kDense, kMerged };
+
+// Shared memory: tile, operations, phases of merged runs, matrices, entries of
+// the merged runs, thread slots of the first stages.  mirror: a second place for
+// the result of a pass with merged runs (or null).
+template <typename R, bool EXACT, Extra EXTRA>
+__global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::type *a, typename Vec2<R>::type *mirror,
+                                                           const __grid_constant__ GateGeom g, const GateOp *gops, const double2 *gmats) {
 	typedef typename Vec2<R>::type V;
 	constexpr unsigned K = tile_bits<R>(), RB = reg_bits<R>(), TB = kThreadBits, kRegs = 1u << RB;
+	constexpr bool MERGED = EXTRA == kMerged;
 	static_assert(RB + TB == K, "one amplitude set per thread");
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	V *s = reinterpret_cast<V *>(smem_raw);
 	GateOp *ops = reinterpret_cast<GateOp *>(smem_raw + (sizeof(V) << K));
 	typedef typename MatElem<R>::type ME;
-	ME *mats = reinterpret_cast<ME *>(ops + g.nops);
-	uint16_t *slots = reinterpret_cast<uint16_t *>(mats + g.nmat);
+	const GateOp *terms = ops + g.nops;
+	ME *mats = reinterpret_cast<ME *>(ops + g.nops + g.nterms);
+	V *dth = reinterpret_cast<V *>(mats + g.nmat), *dti = dth + g.ndiag * kDiagThread * kThreads;
+	uint16_t *slots = reinterpret_cast<uint16_t *>(dti + 2 * g.ndiag * kDiagTile);
 	const unsigned t = threadIdx.x;
-	for(unsigned e = t; e < g.nops * (sizeof(GateOp) / 16); e += blockDim.x)
+	for(unsigned e = t; e < (g.nops + g.nterms) * (sizeof(GateOp) / 16); e += blockDim.x)
 		reinterpret_cast<int4 *>(ops)[e] = reinterpret_cast<const int4 *>(gops)[e];
 	for(unsigned e = t; e < g.nmat; e += blockDim.x) mats[e] = MatElem<R>::make(gmats[e]);
 	// Where this thread's amplitudes sit in shared memory in a stage (register 0).
@@ -440,11 +495,44 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::typ
 		pin += x;
 		pout += y;
 	}
+	const ptrdiff_t other = MERGED && mirror ? mirror - a : 0;
 	__syncthreads();
-	for(uint64_t o = g.o_begin + blockIdx.x; o < g.ntiles; o += gridDim.x) {
-		uint64_t base = o;
+	// Product of the phases of entry e of run d (thread entries, then tile
+	// entries) whose conditions hold.
+	auto entry = [&](unsigned d, unsigned e, uint64_t base) {
+		double re = 1.0, im = 0.0;
+		for(unsigned k = g.term[d][e]; k < g.term[d][e + 1]; ++k) {
+			const GateOp &q = terms[k];
+			if((base & q.omask) != q.omask || (t & q.tmask) != q.tmask) continue;
+			const double x = fma(re, q.cr, -(im * q.ci));
+			im = fma(re, q.ci, im * q.cr);
+			re = x;
+		}
+		V f;
+		f.x = (R)re;
+		f.y = (R)im;
+		return f;
+	};
+	auto tile_base = [&](uint64_t o) {
 #pragma unroll
-		for(unsigned i = 0; i < K; ++i) base = insert0(base, g.lpos[i]);
+		for(unsigned i = 0; i < K; ++i) o = insert0(o, g.lpos[i]);
+		return o;
+	};
+	// The next tile's entries come from one warp while its loads of the current
+	// tile are in flight.
+	const unsigned ntile = MERGED ? g.ndiag * kDiagTile : 0u;
+	auto prepare = [&](uint64_t o, unsigned buf) {
+		if(t < ntile && o < g.ntiles) dti[buf * ntile + t] = entry(t / kDiagTile, kDiagThread + t % kDiagTile, tile_base(o));
+	};
+	if(MERGED) {
+		for(unsigned d = 0; d < g.ndiag; ++d)
+			for(unsigned e = 0; e < kDiagThread; ++e) dth[(d * kDiagThread + e) * kThreads + t] = entry(d, e, 0);
+		prepare(g.o_begin + blockIdx.x, 0);
+		__syncthreads();
+	}
+	unsigned buf = 0;
+	for(uint64_t o = g.o_begin + blockIdx.x; o < g.ntiles; o += gridDim.x, buf ^= 1u) {
+		const uint64_t base = tile_base(o);
 		for(unsigned st = 0; st < g.nstages; ++st) {
 			const bool last = st + 1 == g.nstages;
 			Amps<R> v;
@@ -470,12 +558,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::typ
 			if(st == 0) {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) v[r] = pin[global(g.lpos, r)];
+				if(MERGED) prepare(o + gridDim.x, buf ^ 1u);
 			} else {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) v[r] = s[at(r)];
 			}
 			const unsigned k1 = (unsigned)g.first[st] + g.count[st];
-			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT, DENSE>(ops[k], v, g, mats, base, t);
+			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT, EXTRA == kDense, MERGED>(ops[k], v, g, mats, dth, dti + buf * ntile, base, t);
 			if(last) {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) {
@@ -483,14 +572,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::typ
 						v[r].x *= (R)g.scale;
 						v[r].y *= (R)g.scale;
 					}
-					pout[global(g.opos, r)] = v[r];
+					V *q = pout + global(g.opos, r);
+					*q = v[r];
+					if(MERGED && mirror) q[other] = v[r];
 				}
 			} else {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) s[at(r)] = v[r];
 			}
 			// Between stages, and before the next tile's first stage writes what the last one read.
-			if(g.nstages > 1) __syncthreads();
+			if(g.nstages > 1 || MERGED) __syncthreads();
 		}
 	}
 }
@@ -507,8 +598,9 @@ struct PlanOp {
 };
 
 // The stage plan of a pass; false: it does not fit (another kernel runs it).
-bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, bool exact, GateGeom &g, std::vector<GateOp> &out,
-                std::vector<double> &mats) {
+// `merge`: merge runs of controlled phases; `loose` is the number of them that were not.
+bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, bool exact, bool merge, GateGeom &g, std::vector<GateOp> &out,
+                std::vector<GateOp> &terms, std::vector<double> &mats, unsigned &loose) {
 	if(pass.K != K || pass.ops.empty() || pass.n < K) return false;
 	g = GateGeom{};
 	g.n = pass.n;
@@ -625,6 +717,8 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 	g.nstages = (unsigned)regs.size();
 	if(g.nstages > kMaxStages) return false;
 	out.clear();
+	terms.clear();
+	loose = 0;
 	mats = pass.mats;
 	for(unsigned st = 0; st < g.nstages; ++st) {
 		const bool in = st == 0, outs = st + 1 == g.nstages;
@@ -670,11 +764,57 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 		for(unsigned i = 0; i < RB; ++i) g.rbit[st][i] = (uint8_t)rb[i];
 		for(unsigned k = 0; k < tb.size(); ++k) g.tbit[st][k] = (uint8_t)tb[k];
 		g.first[st] = (uint8_t)out.size();
-		g.count[st] = (uint8_t)of[st].size();
-		for(unsigned k : of[st]) {
+		for(unsigned pos = 0; pos < of[st].size(); ++pos) {
+			const unsigned k = of[st][pos];
 			const PlanOp &q = ops[k];
 			GateOp o{};
 			uint32_t rm = 0, tm = 0;
+			// A run of controlled phases from here on.
+			unsigned end = pos, few = 0;
+			while(merge && end < of[st].size() && ops[of[st][end]].kind == PlanOp::kCP) few += __builtin_popcount(ops[of[st][end++]].pm & r) < 2;
+			if(g.ndiag < kMaxDiag && few >= kDiagMin) {
+				o.code = kCodeDiag;
+				o.rval = (uint16_t)g.ndiag;
+				for(unsigned e = pos; e < end; ++e) {
+					const PlanOp &c = ops[of[st][e]];
+					GateOp x{};
+					x.cr = c.cr;
+					x.ci = c.ci;
+					x.rval = o.rval;
+					uint32_t crm = 0, ctm = 0;
+					for(unsigned i = 0; i < RB; ++i) crm |= ((c.pm >> rb[i]) & 1u) << i;
+					for(unsigned i = 0; i < tb.size(); ++i) ctm |= ((c.pm >> tb[i]) & 1u) << i;
+					if(__builtin_popcount(crm) == 2) {
+						x.code = kCodeCP + crm;
+						x.rval = 0;
+						out.push_back(x);
+						++loose;
+						continue;
+					}
+					x.code = (c.om ? kDiagThread : 0u) + (crm ? 1u + (unsigned)__builtin_ctz(crm) : 0u);
+					if(crm) o.tmask |= (uint16_t)crm;
+					x.tmask = (uint16_t)ctm;
+					x.omask = c.om;
+					if(c.om && ctm) {
+						x.code = kDiagThread + 6u + (unsigned)__builtin_ctz(ctm);
+						x.tmask = 0;
+						o.omask |= ctm;
+					}
+					terms.push_back(x);
+				}
+				out.push_back(o);
+				const auto from = terms.begin() + (g.ndiag ? g.term[g.ndiag - 1][kDiagThread + kDiagTile] : 0);
+				std::stable_sort(from, terms.end(), [](const GateOp &x, const GateOp &y) { return x.code < y.code; });
+				unsigned at = (unsigned)(from - terms.begin());
+				for(unsigned e = 0; e <= kDiagThread + kDiagTile; ++e) {
+					while(at < terms.size() && terms[at].code < e) ++at;
+					g.term[g.ndiag][e] = (uint16_t)at;
+				}
+				++g.ndiag;
+				pos = end - 1;
+				continue;
+			}
+			loose += q.kind == PlanOp::kCP;
 			for(unsigned i = 0; i < RB; ++i) rm |= ((q.pm >> rb[i]) & 1u) << i;
 			for(unsigned i = 0; i < tb.size(); ++i) tm |= ((q.pm >> tb[i]) & 1u) << i;
 			unsigned target = 0, second = 0;
@@ -714,20 +854,27 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 			}
 			out.push_back(o);
 		}
+		g.count[st] = (uint8_t)(out.size() - g.first[st]);
 	}
 	g.nops = (unsigned)out.size();
+	g.nterms = (unsigned)terms.size();
 	g.nmat = (unsigned)(pass.mats.size() / 2);
 	g.scale = std::pow(g.inv, (double)nh);  // of the reference's 1/sqrt(2), rounded as it is: the difference adds up
 	return true;
 }
 
 template <typename R, bool EXACT>
-bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes) {
+bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes, void *mirror, bool merged) {
+	if(merged && (EXACT || sizeof(R) != 8)) return false;
 	constexpr unsigned K = tile_bits<R>();
 	GateGeom g;
 	std::vector<GateOp> ops;
+	std::vector<GateOp> terms;
 	std::vector<double> mats;
-	if(!plan_gates(pass, K, reg_bits<R>(), line_bits<R>(), EXACT, g, ops, mats)) return false;
+	unsigned loose = 0;
+	if(!plan_gates(pass, K, reg_bits<R>(), line_bits<R>(), EXACT, merged, g, ops, terms, mats, loose)) return false;
+	if(merged && (g.ndiag == 0 || loose > kMaxLoose)) return false;
+	ops.insert(ops.end(), terms.begin(), terms.end());
 	const size_t ops_bytes = ops.size() * sizeof(GateOp), mat_bytes = mats.size() * sizeof(double);
 	const size_t need = std::max<size_t>(sizeof(GateOp), ops_bytes + mat_bytes);
 	if(need > dev_prog_bytes) {
@@ -748,13 +895,16 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	if(mat_bytes) std::memcpy(host.data() + ops_bytes, mats.data(), mat_bytes);
 	if(ops_bytes + mat_bytes) upload_async(c, dev_prog, host.data(), ops_bytes + mat_bytes, "gate pass program upload");
 	typedef typename Vec2<R>::type V;
-	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(typename MatElem<R>::type) + sizeof(uint16_t) * kThreads * std::min(g.nstages, kSlotStages);
-	auto kern = mats.empty() ? k_gate_pass<R, EXACT, false> : k_gate_pass<R, EXACT, true>;
+	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(typename MatElem<R>::type) +
+	                    g.ndiag * (kDiagThread * kThreads + 2 * kDiagTile) * sizeof(V) + sizeof(uint16_t) * kThreads * std::min(g.nstages, kSlotStages);
+	auto kern = mats.empty() ? k_gate_pass<R, EXACT, kPlain> : k_gate_pass<R, EXACT, kDense>;
+	if constexpr(!EXACT && sizeof(R) == 8)
+		if(merged) kern = k_gate_pass<R, EXACT, kMerged>;
 	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gate pass smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem), "gate pass occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));
-	kern<<<(unsigned)grid, kThreads, smem, c.stream>>>(static_cast<V *>(a), g, static_cast<const GateOp *>(dev_prog),
+	kern<<<(unsigned)grid, kThreads, smem, c.stream>>>(static_cast<V *>(a), static_cast<V *>(mirror), g, static_cast<const GateOp *>(dev_prog),
 	                                                 reinterpret_cast<const double2 *>(static_cast<unsigned char *>(dev_prog) + ops_bytes));
 	check_cuda(cudaGetLastError(), "gate pass");
 	if(c.launches) ++*c.launches;
@@ -763,10 +913,11 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 
 }  // namespace
 
-bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes) {
-	if(prec == TMFQS_FP32) return run_gate_pass<float, false>(c, a, pass, dev_prog, dev_prog_bytes);
-	return exact ? run_gate_pass<double, true>(c, a, pass, dev_prog, dev_prog_bytes)
-	             : run_gate_pass<double, false>(c, a, pass, dev_prog, dev_prog_bytes);
+bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes,
+                      void *mirror, bool merged) {
+	if(prec == TMFQS_FP32) return run_gate_pass<float, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
+	return exact ? run_gate_pass<double, true>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged)
+	             : run_gate_pass<double, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
 }
 
 }  // namespace tqb

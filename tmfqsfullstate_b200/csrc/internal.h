@@ -180,9 +180,11 @@ struct FusedPass {
 void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
                        size_t &dev_prog_bytes);
 // Any fused pass on a full tile as register stages (gate_pass.cu); false
-// (nothing launched) when its plan does not fit.
+// (nothing launched) when its plan does not fit.  With `merged` (fast complex128
+// form) only a pass nearly all of whose controlled phases merge, and with
+// `mirror` (a state-sized buffer) its result is written there too.
 bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
-                      size_t &dev_prog_bytes);
+                      size_t &dev_prog_bytes, void *mirror = nullptr, bool merged = false);
 
 // Uploads the program of an exact register-stage pass into `dev_prog` ahead
 // of its launches (the tile ranges of one pass share it); false when the pass
