@@ -43,7 +43,6 @@ namespace {
 constexpr unsigned kMaxRB = 5;
 constexpr unsigned kMaxK = 13;
 constexpr unsigned kMaxStages = 64;
-constexpr unsigned kSlotStages = 8;  // stages whose thread slots are kept in shared memory
 constexpr unsigned kMaxOps = 240;
 
 // Tiles of 64 KiB.
@@ -51,12 +50,21 @@ template <typename R>
 constexpr unsigned tile_bits() {
 	return sizeof(R) == 8 ? 12u : 13u;
 }
-// Register bits per stage: 16 complex128 or 32 complex64 amplitudes per thread (64 registers), 256 threads.
+// Register bits per stage: 16 complex128 or 32 complex64 amplitudes per thread
+// (64 registers), 256 threads.  Passes of no more tiles than SMs leave most of the
+// chip idle and wait on each thread's chain of operations: half the amplitudes per
+// thread there (QFT-12 complex128, 84 operations: 38 -> 31 us; circuit of 60 on 14
+// qubits 86 -> 73 us in all).
 template <typename R>
 constexpr unsigned reg_bits() {
 	return sizeof(R) == 8 ? 4u : 5u;
 }
-constexpr unsigned kThreadBits = 8, kThreads = 1u << kThreadBits;
+template <typename R>
+constexpr unsigned small_bits() {
+	return reg_bits<R>() - 1u;
+}
+constexpr unsigned kThreadBits = 8, kThreads = 1u << kThreadBits;  // of the large form
+constexpr unsigned kMaxTB = 9;
 // Index bits of a 128-byte line: lanes in stages that touch HBM, and the shared-memory slot bits that pick a bank group.
 template <typename R>
 constexpr unsigned line_bits() {
@@ -88,6 +96,23 @@ struct GateOp {
 	double cr, ci;
 };
 
+// A stage as the kernel uses it, in shared memory: the slot of thread index t
+// (three nibbles, XORed) and of each register bit, and its operations.
+struct StageSlots {
+	uint16_t reg[8];
+	uint16_t first, end, pad[6];
+	uint16_t nib[3][16];
+};
+
+// An operation in the kernel's precision, in shared memory.
+template <typename R>
+struct alignas(16) OpS {
+	uint32_t code;
+	uint16_t tmask, rval;
+	uint64_t omask;
+	R cr, ci;
+};
+
 struct GateGeom {
 	unsigned n, nstages, nops, nmat;  // nmat: complex matrix elements of the dense gates
 	unsigned ndiag, nterms;           // merged phase runs, and the phases in them (after the operations)
@@ -98,7 +123,7 @@ struct GateGeom {
 	uint8_t lpos[kMaxK], opos[kMaxK];  // index bit of a tile bit when loaded and when stored
 	uint8_t first[kMaxStages], count[kMaxStages];
 	uint8_t rbit[kMaxStages][kMaxRB];        // tile bit of register bit i
-	uint8_t tbit[kMaxStages][kThreadBits];  // tile bit of thread index bit k
+	uint8_t tbit[kMaxStages][kMaxTB];  // tile bit of thread index bit k
 };
 
 // Non-sign bits of an amplitude: zero exactly for +-0 +- 0i (integer units, not the FP64 pipe).
@@ -108,9 +133,9 @@ __device__ __forceinline__ unsigned nonzero_bits(double2 x) {
 }
 
 // A thread's amplitudes of a stage.
-template <typename R>
+template <typename R, unsigned RB>
 struct Amps {
-	static constexpr unsigned kRegs = 1u << reg_bits<R>();
+	static constexpr unsigned kRegs = 1u << RB;
 	typename Vec2<R>::type v[kRegs];
 	__device__ __forceinline__ typename Vec2<R>::type &operator[](unsigned r) { return v[r]; }
 };
@@ -127,8 +152,8 @@ __device__ __forceinline__ unsigned maybe_zero(double2 x) {
 	return (unsigned)(__double2hiint(x.x) | __double2hiint(x.y)) & 0x7fffffffu;
 }
 
-template <typename R, bool EXACT, unsigned I>
-__device__ __forceinline__ void op_h(Amps<R> &v, R inv) {
+template <typename R, unsigned RB, bool EXACT, unsigned I>
+__device__ __forceinline__ void op_h(Amps<R, RB> &v, R inv) {
 	typedef typename Vec2<R>::type V;
 	auto bfly = [&](V &x, V &y) {
 		V o0 = cadd(x, y), o1 = csub(x, y);
@@ -141,7 +166,7 @@ __device__ __forceinline__ void op_h(Amps<R> &v, R inv) {
 		x = o0;
 		y = o1;
 	};
-	constexpr unsigned kRegs = Amps<R>::kRegs;
+	constexpr unsigned kRegs = Amps<R, RB>::kRegs;
 	if constexpr(EXACT) {
 		// An all-zero pair is left as it is (dense_state_backend.cpp:265).
 		unsigned least = ~0u;
@@ -161,9 +186,9 @@ __device__ __forceinline__ void op_h(Amps<R> &v, R inv) {
 }
 
 // X on register bit I of the pairs whose register bit C is set (C == I: all).
-template <typename R, bool EXACT, unsigned I, unsigned C>
-__device__ __forceinline__ void op_x(Amps<R> &v, bool on) {
-	constexpr unsigned kRegs = Amps<R>::kRegs;
+template <typename R, unsigned RB, bool EXACT, unsigned I, unsigned C>
+__device__ __forceinline__ void op_x(Amps<R, RB> &v, bool on) {
+	constexpr unsigned kRegs = Amps<R, RB>::kRegs;
 #pragma unroll
 	for(unsigned r = 0; r < kRegs; ++r) {
 		if(((r >> I) & 1u) || (C != I && !((r >> C) & 1u))) continue;
@@ -178,9 +203,9 @@ __device__ __forceinline__ void op_x(Amps<R> &v, bool on) {
 }
 
 // Phase on the registers that have all bits of M.
-template <typename R, bool EXACT, unsigned M>
-__device__ __forceinline__ void op_cp(Amps<R> &v, R pr, R pi) {
-	constexpr unsigned kRegs = Amps<R>::kRegs;
+template <typename R, unsigned RB, bool EXACT, unsigned M>
+__device__ __forceinline__ void op_cp(Amps<R, RB> &v, R pr, R pi) {
+	constexpr unsigned kRegs = Amps<R, RB>::kRegs;
 	unsigned least = ~0u;
 	if constexpr(EXACT) {
 #pragma unroll
@@ -245,12 +270,12 @@ __device__ __forceinline__ void cfma(double2 g, double2 x, double2, double2 &o) 
 }
 
 // Dense gate on register bit I: the unrolled formula of gate_block_apply.h:117-140.
-template <typename R, bool EXACT, unsigned I>
-__device__ __forceinline__ void op_u1(Amps<R> &v, const typename MatElem<R>::type *m) {
+template <typename R, unsigned RB, bool EXACT, unsigned I>
+__device__ __forceinline__ void op_u1(Amps<R, RB> &v, const typename MatElem<R>::type *m) {
 	typedef typename Vec2<R>::type V;
 	const auto g00 = m[0], g01 = m[1], g10 = m[2], g11 = m[3];
 #pragma unroll
-	for(unsigned r = 0; r < Amps<R>::kRegs; ++r) {
+	for(unsigned r = 0; r < Amps<R, RB>::kRegs; ++r) {
 		if((r >> I) & 1u) continue;
 		const V x = v[r], y = v[r | (1u << I)];
 		if constexpr(EXACT) {
@@ -276,10 +301,10 @@ __device__ __forceinline__ void op_u1(Amps<R> &v, const typename MatElem<R>::typ
 // Dense gate on register bits A (more significant) and B: row sums term by term
 // (gate_block_apply.h:165-176); all-zero blocks are left alone.  Fast forms: two
 // blocks per matrix element loaded.
-template <typename R, bool EXACT, unsigned A, unsigned B>
-__device__ __forceinline__ void op_u2(Amps<R> &v, const typename MatElem<R>::type *m) {
+template <typename R, unsigned RB, bool EXACT, unsigned A, unsigned B>
+__device__ __forceinline__ void op_u2(Amps<R, RB> &v, const typename MatElem<R>::type *m) {
 	typedef typename Vec2<R>::type V;
-	constexpr unsigned RB = reg_bits<R>(), mask = (1u << A) | (1u << B);
+	constexpr unsigned mask = (1u << A) | (1u << B);
 	// Register of index c of block b.
 	auto at = [](unsigned b, unsigned c) {
 		unsigned r = 0, k = 0;
@@ -289,7 +314,7 @@ __device__ __forceinline__ void op_u2(Amps<R> &v, const typename MatElem<R>::typ
 	};
 	if constexpr(EXACT) {
 #pragma unroll
-		for(unsigned b = 0; b < Amps<R>::kRegs / 4; ++b) {
+		for(unsigned b = 0; b < Amps<R, RB>::kRegs / 4; ++b) {
 			V o[4];
 			if((nonzero_bits(v[at(b, 0)]) | nonzero_bits(v[at(b, 1)]) | nonzero_bits(v[at(b, 2)]) | nonzero_bits(v[at(b, 3)])) == 0u) continue;
 #pragma unroll
@@ -310,7 +335,7 @@ __device__ __forceinline__ void op_u2(Amps<R> &v, const typename MatElem<R>::typ
 		}
 	} else {
 #pragma unroll
-		for(unsigned b = 0; b < Amps<R>::kRegs / 4; b += 2) {
+		for(unsigned b = 0; b < Amps<R, RB>::kRegs / 4; b += 2) {
 			V o[2][4];
 #pragma unroll
 			for(unsigned k = 0; k < 2; ++k)
@@ -348,11 +373,11 @@ __device__ __forceinline__ V cprod(V a, V b) {
 }
 
 // A merged run: dth this run's thread entries (per thread), dti its tile entries.
-template <typename R>
-__device__ __forceinline__ void op_diag(const GateOp &op, Amps<R> &v, const typename Vec2<R>::type *dth, const typename Vec2<R>::type *dti,
+template <typename R, unsigned RB>
+__device__ __forceinline__ void op_diag(const OpS<R> &op, Amps<R, RB> &v, const typename Vec2<R>::type *dth, const typename Vec2<R>::type *dti,
                                         unsigned t) {
 	typedef typename Vec2<R>::type V;
-	constexpr unsigned RB = reg_bits<R>(), kRegs = Amps<R>::kRegs;
+	constexpr unsigned kRegs = Amps<R, RB>::kRegs;
 	V p = cprod(dth[t], dti[0]);
 	for(unsigned m = (unsigned)op.omask; m; m &= m - 1u) {
 		const unsigned k = __ffs(m) - 1;
@@ -370,12 +395,11 @@ __device__ __forceinline__ void op_diag(const GateOp &op, Amps<R> &v, const type
 	}
 }
 
-template <typename R, bool EXACT, bool DENSE, bool MERGED>
-__device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateGeom &g, const typename MatElem<R>::type *mats,
+template <typename R, unsigned RB, bool EXACT, bool DENSE, bool MERGED>
+__device__ __forceinline__ void run_op(const OpS<R> &op, Amps<R, RB> &v, const GateGeom &g, const typename MatElem<R>::type *mats,
                                        const typename Vec2<R>::type *dth, const typename Vec2<R>::type *dti, uint64_t base, unsigned t) {
-	constexpr unsigned RB = reg_bits<R>();
 	if(MERGED && op.code == kCodeDiag) {
-		op_diag<R>(op, v, dth + op.rval * kDiagThread * kThreads, dti + op.rval * kDiagTile, t);
+		op_diag<R, RB>(op, v, dth + op.rval * kDiagThread * kThreads, dti + op.rval * kDiagTile, t);
 		return;
 	}
 	if(DENSE && op.code >= kCodeU1) {
@@ -383,11 +407,11 @@ __device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateG
 		switch(op.code) {
 #define TQB_U1(I)                                                         \
 	case kCodeU1 + I:                                                     \
-		if constexpr(DENSE && I < RB) op_u1<R, EXACT, I < RB ? I : 0u>(v, m);      \
+		if constexpr(DENSE && I < RB) op_u1<R, RB, EXACT, I < RB ? I : 0u>(v, m);      \
 		return;
 #define TQB_U2(A, B)                                                                                    \
 	case kCodeU2 + 5 * A + B:                                                                           \
-		if constexpr(DENSE && A < RB && B < RB && (EXACT || A > B)) op_u2<R, EXACT, A < RB ? A : 0u, B < RB ? B : 0u>(v, m); \
+		if constexpr(DENSE && A < RB && B < RB && (EXACT || A > B)) op_u2<R, RB, EXACT, A < RB ? A : 0u, B < RB ? B : 0u>(v, m); \
 		return;
 			TQB_U1(0) TQB_U1(1) TQB_U1(2) TQB_U1(3) TQB_U1(4)
 			TQB_U2(0, 1) TQB_U2(0, 2) TQB_U2(0, 3) TQB_U2(1, 0) TQB_U2(1, 2) TQB_U2(1, 3)
@@ -399,9 +423,9 @@ __device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateG
 		}
 	}
 	if(op.code == kCodeFlip) {
-		const unsigned at = (base & g.outer) == op.omask && t == op.tmask ? op.rval : Amps<R>::kRegs;
+		const unsigned at = (base & g.outer) == op.omask && t == op.tmask ? op.rval : Amps<R, RB>::kRegs;
 #pragma unroll
-		for(unsigned r = 0; r < Amps<R>::kRegs; ++r) {
+		for(unsigned r = 0; r < Amps<R, RB>::kRegs; ++r) {
 			v[r].x = r == at ? -v[r].x : v[r].x;
 			v[r].y = r == at ? -v[r].y : v[r].y;
 		}
@@ -409,35 +433,31 @@ __device__ __forceinline__ void run_op(const GateOp &op, Amps<R> &v, const GateG
 	}
 	if((base & op.omask) != op.omask) return;
 	const bool on = (t & op.tmask) == op.tmask;
-	const R inv = (R)g.inv;
+	const R inv = (R)g.inv, pr = op.cr, pi = op.ci;
 	switch(op.code) {
 #define TQB_H(I)                                                          \
 	case kCodeH + I:                                                      \
-		if constexpr(I < RB) op_h<R, EXACT, I < RB ? I : 0u>(v, inv);     \
+		if constexpr(I < RB) op_h<R, RB, EXACT, I < RB ? I : 0u>(v, inv);     \
 		return;
 #define TQB_XC(I, C)                                                                                       \
 	case kCodeX + 5 * I + C:                                                                               \
-		if constexpr(I < RB && C < RB) op_x<R, EXACT, I < RB ? I : 0u, C < RB ? C : 0u>(v, on);            \
+		if constexpr(I < RB && C < RB) op_x<R, RB, EXACT, I < RB ? I : 0u, C < RB ? C : 0u>(v, on);            \
 		return;
 #define TQB_X(I) TQB_XC(I, 0) TQB_XC(I, 1) TQB_XC(I, 2) TQB_XC(I, 3) TQB_XC(I, 4)
 		TQB_H(0) TQB_H(1) TQB_H(2) TQB_H(3) TQB_H(4)
 		TQB_X(0) TQB_X(1) TQB_X(2) TQB_X(3) TQB_X(4)
-#undef TQB_H
-#undef TQB_X
-#undef TQB_XC
-		default: break;
-	}
-	if(!on) return;
-	const R pr = (R)op.cr, pi = (R)op.ci;
-	switch(op.code) {
-#define TQB_CP(M)                                                                     \
-	case kCodeCP + M:                                                                 \
-		if constexpr(M < (1u << RB)) op_cp<R, EXACT, M < (1u << RB) ? M : 0u>(v, pr, pi); \
+#define TQB_CP(M)                                                                                    \
+	case kCodeCP + M:                                                                                \
+		if constexpr(M < (1u << RB))                                                                 \
+			if(on) op_cp<R, RB, EXACT, M < (1u << RB) ? M : 0u>(v, pr, pi);                          \
 		return;
 		TQB_CP(0) TQB_CP(1) TQB_CP(2) TQB_CP(3) TQB_CP(4) TQB_CP(5) TQB_CP(6) TQB_CP(8) TQB_CP(9) TQB_CP(10) TQB_CP(12)
 		TQB_CP(16) TQB_CP(17) TQB_CP(18) TQB_CP(20) TQB_CP(24)
+		default: return;
+#undef TQB_H
+#undef TQB_X
+#undef TQB_XC
 #undef TQB_CP
-		default: break;
 	}
 }
 
@@ -452,36 +472,45 @@ __device__ __forceinline__ unsigned slot_of(unsigned b) {
 // What a pass holds beside the plain operations: each costs the others registers.
 enum Extra { kPlain, kDense, kMerged };
 
-// Shared memory: tile, operations, phases of merged runs, matrices, entries of
-// the merged runs, thread slots of the first stages.  mirror: a second place for
+// Shared memory: tile, operations, phases of merged runs, stages, matrices,
+// entries of the merged runs.  mirror: a second place for
 // the result of a pass with merged runs (or null).
-template <typename R, bool EXACT, Extra EXTRA>
-__global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::type *a, typename Vec2<R>::type *mirror,
+template <typename R, unsigned RB, bool EXACT, Extra EXTRA>
+__global__ void __launch_bounds__(1u << (tile_bits<R>() - RB), RB == small_bits<R>() ? 1 : 2) k_gate_pass(typename Vec2<R>::type *a, typename Vec2<R>::type *mirror,
                                                            const __grid_constant__ GateGeom g, const GateOp *gops, const double2 *gmats) {
 	typedef typename Vec2<R>::type V;
-	constexpr unsigned K = tile_bits<R>(), RB = reg_bits<R>(), TB = kThreadBits, kRegs = 1u << RB;
+	constexpr unsigned K = tile_bits<R>(), TB = K - RB, kThreads = 1u << TB, kRegs = 1u << RB;
 	constexpr bool MERGED = EXTRA == kMerged;
-	static_assert(RB + TB == K, "one amplitude set per thread");
+	static_assert(!MERGED || TB == kThreadBits, "entries of merged runs are per thread of the large form");
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	V *s = reinterpret_cast<V *>(smem_raw);
-	GateOp *ops = reinterpret_cast<GateOp *>(smem_raw + (sizeof(V) << K));
+	OpS<R> *ops = reinterpret_cast<OpS<R> *>(smem_raw + (sizeof(V) << K));
+	GateOp *terms = reinterpret_cast<GateOp *>(ops + g.nops);
+	StageSlots *stages = reinterpret_cast<StageSlots *>(terms + g.nterms);
 	typedef typename MatElem<R>::type ME;
-	const GateOp *terms = ops + g.nops;
-	ME *mats = reinterpret_cast<ME *>(ops + g.nops + g.nterms);
+	ME *mats = reinterpret_cast<ME *>(stages + g.nstages);
 	V *dth = reinterpret_cast<V *>(mats + g.nmat), *dti = dth + g.ndiag * kDiagThread * kThreads;
-	uint16_t *slots = reinterpret_cast<uint16_t *>(dti + 2 * g.ndiag * kDiagTile);
 	const unsigned t = threadIdx.x;
-	for(unsigned e = t; e < (g.nops + g.nterms) * (sizeof(GateOp) / 16); e += blockDim.x)
-		reinterpret_cast<int4 *>(ops)[e] = reinterpret_cast<const int4 *>(gops)[e];
+	for(unsigned e = t; e < g.nops; e += blockDim.x) {
+		const GateOp q = gops[e];
+		ops[e] = OpS<R>{q.code, q.tmask, q.rval, q.omask, (R)q.cr, (R)q.ci};
+	}
+	for(unsigned e = t; e < g.nterms; e += blockDim.x) terms[e] = gops[g.nops + e];
 	for(unsigned e = t; e < g.nmat; e += blockDim.x) mats[e] = MatElem<R>::make(gmats[e]);
-	// Where this thread's amplitudes sit in shared memory in a stage (register 0).
-	auto thread_slot = [&](unsigned st) {
-		unsigned x = 0;
-#pragma unroll
-		for(unsigned k = 0; k < TB; ++k) x ^= (t >> k) & 1u ? slot_of<R>(g.tbit[st][k]) : 0u;
-		return x;
-	};
-	for(unsigned st = 0; st < min(g.nstages, kSlotStages); ++st) slots[st * kThreads + t] = (uint16_t)thread_slot(st);
+	for(unsigned e = t; e < g.nstages * 64u; e += blockDim.x) {
+		const unsigned st = e >> 6, i = e & 63u;
+		if(i < 48u) {
+			unsigned x = 0;
+			for(unsigned k = 0; k < 4; ++k)
+				if(4 * (i >> 4) + k < TB && ((i >> k) & 1u)) x ^= slot_of<R>(g.tbit[st][4 * (i >> 4) + k]);
+			stages[st].nib[i >> 4][i & 15u] = (uint16_t)x;
+		} else if(i < 48u + RB) {
+			stages[st].reg[i - 48u] = (uint16_t)slot_of<R>(g.rbit[st][i - 48u]);
+		} else if(i == 60u) {
+			stages[st].first = g.first[st];
+			stages[st].end = (uint16_t)(g.first[st] + g.count[st]);
+		}
+	}
 	// And in HBM, when the tile is loaded and stored.
 	V *pin = a, *pout = a;
 	{
@@ -535,11 +564,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::typ
 		const uint64_t base = tile_base(o);
 		for(unsigned st = 0; st < g.nstages; ++st) {
 			const bool last = st + 1 == g.nstages;
-			Amps<R> v;
-			const unsigned slot = st < kSlotStages ? slots[st * kThreads + t] : thread_slot(st);
+			Amps<R, RB> v;
+			// Where this thread's amplitudes sit in shared memory.
+			const StageSlots &sl = stages[st];
+			const unsigned slot = (unsigned)sl.nib[0][t & 15u] ^ sl.nib[1][(t >> 4) & 15u] ^ (TB > 8 ? sl.nib[2][t >> 8] : 0u);
 			unsigned ro[RB];
 #pragma unroll
-			for(unsigned i = 0; i < RB; ++i) ro[i] = slot_of<R>(g.rbit[st][i]);
+			for(unsigned i = 0; i < RB; ++i) ro[i] = sl.reg[i];
 			auto at = [&](unsigned r) {
 				unsigned x = 0;
 #pragma unroll
@@ -563,8 +594,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_pass(typename Vec2<R>::typ
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) v[r] = s[at(r)];
 			}
-			const unsigned k1 = (unsigned)g.first[st] + g.count[st];
-			for(unsigned k = g.first[st]; k < k1; ++k) run_op<R, EXACT, EXTRA == kDense, MERGED>(ops[k], v, g, mats, dth, dti + buf * ntile, base, t);
+			const unsigned k1 = sl.end;
+			for(unsigned k = sl.first; k < k1; ++k) run_op<R, RB, EXACT, EXTRA == kDense, MERGED>(ops[k], v, g, mats, dth, dti + buf * ntile, base, t);
 			if(last) {
 #pragma unroll
 				for(unsigned r = 0; r < kRegs; ++r) {
@@ -863,7 +894,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 	return true;
 }
 
-template <typename R, bool EXACT>
+template <typename R, unsigned RB, bool EXACT>
 bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes, void *mirror, bool merged) {
 	if(merged && (EXACT || sizeof(R) != 8)) return false;
 	constexpr unsigned K = tile_bits<R>();
@@ -872,7 +903,7 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	std::vector<GateOp> terms;
 	std::vector<double> mats;
 	unsigned loose = 0;
-	if(!plan_gates(pass, K, reg_bits<R>(), line_bits<R>(), EXACT, merged, g, ops, terms, mats, loose)) return false;
+	if(!plan_gates(pass, K, RB, line_bits<R>(), EXACT, merged, g, ops, terms, mats, loose)) return false;
 	if(merged && (g.ndiag == 0 || loose > kMaxLoose)) return false;
 	ops.insert(ops.end(), terms.begin(), terms.end());
 	const size_t ops_bytes = ops.size() * sizeof(GateOp), mat_bytes = mats.size() * sizeof(double);
@@ -895,29 +926,38 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	if(mat_bytes) std::memcpy(host.data() + ops_bytes, mats.data(), mat_bytes);
 	if(ops_bytes + mat_bytes) upload_async(c, dev_prog, host.data(), ops_bytes + mat_bytes, "gate pass program upload");
 	typedef typename Vec2<R>::type V;
-	const size_t smem = (sizeof(V) << K) + ops_bytes + g.nmat * sizeof(typename MatElem<R>::type) +
-	                    g.ndiag * (kDiagThread * kThreads + 2 * kDiagTile) * sizeof(V) + sizeof(uint16_t) * kThreads * std::min(g.nstages, kSlotStages);
-	auto kern = mats.empty() ? k_gate_pass<R, EXACT, kPlain> : k_gate_pass<R, EXACT, kDense>;
-	if constexpr(!EXACT && sizeof(R) == 8)
-		if(merged) kern = k_gate_pass<R, EXACT, kMerged>;
+	const size_t smem = (sizeof(V) << K) + g.nops * sizeof(OpS<R>) + g.nterms * sizeof(GateOp) + g.nstages * sizeof(StageSlots) +
+	                    g.nmat * sizeof(typename MatElem<R>::type) + g.ndiag * (kDiagThread * kThreads + 2 * kDiagTile) * sizeof(V);
+	constexpr unsigned threads = 1u << (K - RB);
+	auto kern = mats.empty() ? k_gate_pass<R, RB, EXACT, kPlain> : k_gate_pass<R, RB, EXACT, kDense>;
+	if constexpr(!EXACT && sizeof(R) == 8 && RB != small_bits<R>())
+		if(merged) kern = k_gate_pass<R, RB, EXACT, kMerged>;
 	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gate pass smem");
 	int per_sm = 1;
-	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem), "gate pass occupancy");
+	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem), "gate pass occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));
-	kern<<<(unsigned)grid, kThreads, smem, c.stream>>>(static_cast<V *>(a), static_cast<V *>(mirror), g, static_cast<const GateOp *>(dev_prog),
+	kern<<<(unsigned)grid, threads, smem, c.stream>>>(static_cast<V *>(a), static_cast<V *>(mirror), g, static_cast<const GateOp *>(dev_prog),
 	                                                 reinterpret_cast<const double2 *>(static_cast<unsigned char *>(dev_prog) + ops_bytes));
 	check_cuda(cudaGetLastError(), "gate pass");
 	if(c.launches) ++*c.launches;
 	return true;
 }
 
+template <typename R, bool EXACT>
+bool pick_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes, void *mirror, bool merged) {
+	const uint64_t tiles = pass.n >= tile_bits<R>() ? 1ull << (pass.n - tile_bits<R>()) : 0;
+	if(!merged && tiles <= (uint64_t)c.num_sms && run_gate_pass<R, small_bits<R>(), EXACT>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged))
+		return true;
+	return run_gate_pass<R, reg_bits<R>(), EXACT>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
+}
+
 }  // namespace
 
 bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes,
                       void *mirror, bool merged) {
-	if(prec == TMFQS_FP32) return run_gate_pass<float, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
-	return exact ? run_gate_pass<double, true>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged)
-	             : run_gate_pass<double, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
+	if(prec == TMFQS_FP32) return pick_gate_pass<float, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
+	return exact ? pick_gate_pass<double, true>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged)
+	             : pick_gate_pass<double, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
 }
 
 }  // namespace tqb
