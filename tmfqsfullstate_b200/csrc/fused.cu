@@ -1626,10 +1626,13 @@ bool prepare_fused_pass(const LaunchCtx &c, int prec, const FusedPass &pass, voi
 	return run_fused_stages<double>(c, nullptr, pass, dev_prog, dev_prog_bytes, true);
 }
 
-void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
-                       size_t &dev_prog_bytes) {
-	if(prec == TMFQS_FP64 && run_fused_stages<double>(c, a, pass, dev_prog, dev_prog_bytes)) return;
-	if(launch_gate_pass(c, prec, exact, a, pass, dev_prog, dev_prog_bytes)) return;
+bool launch_fused_stages(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
+                         size_t &dev_prog_bytes) {
+	return prec == TMFQS_FP64 && run_fused_stages<double>(c, a, pass, dev_prog, dev_prog_bytes);
+}
+
+void launch_fused_ops(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
+                      size_t &dev_prog_bytes) {
 	if(prec == TMFQS_FP64) run_fused<double>(c, a, pass, dev_prog, dev_prog_bytes);
 	else run_fused<float>(c, a, pass, dev_prog, dev_prog_bytes);
 }

@@ -960,4 +960,11 @@ bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const F
 	             : pick_gate_pass<double, false>(c, a, pass, dev_prog, dev_prog_bytes, mirror, merged);
 }
 
+void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
+                       size_t &dev_prog_bytes) {
+	if(launch_fused_stages(c, prec, a, pass, dev_prog, dev_prog_bytes)) return;
+	if(launch_gate_pass(c, prec, exact, a, pass, dev_prog, dev_prog_bytes)) return;
+	launch_fused_ops(c, prec, a, pass, dev_prog, dev_prog_bytes);
+}
+
 }  // namespace tqb

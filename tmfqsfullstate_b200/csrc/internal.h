@@ -185,6 +185,13 @@ void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const 
 // `mirror` (a state-sized buffer) its result is written there too.
 bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
                       size_t &dev_prog_bytes, void *mirror = nullptr, bool merged = false);
+// The other two kernels of launch_fused_pass (fused.cu): the exact register
+// stages of Hadamards and their chains (false: nothing launched), and the
+// op-by-op pass, which takes every program.
+bool launch_fused_stages(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
+                         size_t &dev_prog_bytes);
+void launch_fused_ops(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
+                      size_t &dev_prog_bytes);
 
 // Uploads the program of an exact register-stage pass into `dev_prog` ahead
 // of its launches (the tile ranges of one pass share it); false when the pass
