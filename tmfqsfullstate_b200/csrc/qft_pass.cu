@@ -452,8 +452,13 @@ __device__ __forceinline__ void qft_tail(const V *tile, V *dst, unsigned T, unsi
 // thread's first amplitude per stage [nstages][nthr], and one row of per-tile
 // factors per ring slot.  Everything is derived here from the geometry: the
 // launch needs no device program.
-template <typename R, int RB, bool TM>
-__global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type), RB), 1)
+//
+// ONE: a single tile buffer and two blocks per SM instead of a ring of three and
+// one block: a pass of three stages spends longer in each tile than its bytes
+// take, its few warps in step (all at their shared-memory accesses, then all at
+// their arithmetic), and two blocks out of step fill each other's gaps.
+template <typename R, int RB, bool TM, bool ONE>
+__global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type), RB), ONE ? 2 : 1)
 	k_qft_pass(typename Vec2<R>::type *a, const __grid_constant__ QftGeom g, const __grid_constant__ CUtensorMap tmap,
 	           int *err) {
 	typedef typename Vec2<R>::type V;
@@ -508,7 +513,7 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 		}
 	};
 	uint64_t o = blockIdx.x;
-	for(unsigned k = 0; k + 1 < g.slots; ++k) prefetch(o + (uint64_t)k * gridDim.x, k);
+	for(unsigned k = 0; k < (ONE ? 1u : g.slots - 1u); ++k) prefetch(o + (uint64_t)k * gridDim.x, k);
 
 	// Per-thread tables (once per launch), and the global offset of the
 	// thread's first amplitude in the last stage (direct stores).
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 			// Past the first stage's barrier every thread is done with the
 			// previous tile's buffer: the next copies go there.  (A pass of one
 			// direct stage has no barrier of its own: take one.)
-			if(st == 0) {
+			if(!ONE && st == 0) {
 				if(last && direct) __syncthreads();
 				prefetch(o + (uint64_t)(g.slots - 1) * gridDim.x, slot == 0 ? g.slots - 1 : slot - 1);
 			}
@@ -578,6 +583,10 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 #pragma unroll
 			for(unsigned i = 0; i < kGranules; ++i)
 				*reinterpret_cast<float4 *>(dst + i * g.istride) = *reinterpret_cast<const float4 *>(src + i * gstep);
+		}
+		if constexpr(ONE) {
+			__syncthreads();  // the tile is read no more
+			prefetch(o + gridDim.x, 0);
 		}
 		if(++slot == g.slots) {
 			slot = 0;
@@ -976,17 +985,27 @@ bool run_qft(const LaunchCtx &c, void *a, const FusedPass &pass, const std::vect
 	check_cuda(cudaGetDevice(&dev), "qft device");
 	check_cuda(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "qft smem limit");
 	g.slots = smem_for(3) <= (size_t)max_optin ? 3u : 2u;
+	// Three and more stages: two blocks per SM with one buffer each, where the
+	// tiles keep both busy (four and more to an SM).  Ring against two blocks, last
+	// pass of a QFT: complex64 at 30, 29 and 23 qubits 4128, 2073 and 83 us against
+	// 3850, 1934 and 46; complex128 at 29, 27 and 25 4100, 1128 and 230 against 3730,
+	// 1070 and 224.  Passes of two stages have room for the bytes of a tile and
+	// keep the ring (complex128 at 23 qubits 70 us against 72).
+	const bool one = !g.tma && g.nstages >= 3 && smem_for(1) + 1024 <= (size_t)max_optin / 2 &&
+	                 g.ntiles >= 4ull * (uint64_t)c.num_sms;
+	if(one) g.slots = 1;
 	const size_t smem = smem_for(g.slots);
 	if(smem > (size_t)max_optin) return false;
 	CUtensorMap tmap;
 	std::memset(&tmap, 0, sizeof(tmap));
 	if(g.tma && !encode_tile_map(tmap, a, g)) g.tma = 0;  // no encoder: per-thread copies (same swizzle)
-	void (*kern)(V *, const QftGeom, const CUtensorMap, int *) = k_qft_pass<R, RB, false>;
+	void (*kern)(V *, const QftGeom, const CUtensorMap, int *) =
+		one ? k_qft_pass<R, RB, false, true> : k_qft_pass<R, RB, false, false>;
 	if constexpr(sizeof(V) == 8) {  // tensor-map tiles: complex64 only
-		if(g.tma) kern = k_qft_pass<R, RB, true>;
+		if(g.tma) kern = k_qft_pass<R, RB, true, false>;
 	}
 	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "qft smem");
-	const uint64_t grid = std::min<uint64_t>(g.ntiles, (uint64_t)c.num_sms);
+	const uint64_t grid = std::min<uint64_t>(g.ntiles, (uint64_t)c.num_sms * (one ? 2u : 1u));
 	kern<<<(unsigned)grid, nthr, smem, c.stream>>>(static_cast<V *>(a), g, tmap, c.err);
 	check_cuda(cudaGetLastError(), "qft pass");
 	if(c.launches) ++*c.launches;
