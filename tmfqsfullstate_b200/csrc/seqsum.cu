@@ -25,9 +25,9 @@
 // walk block alone.
 //
 // Bound: HBM, one read of the state, and behind it the walk, a serial chain of
-// about 10 us per binade crossing.  Total probability, complex128, n = 28:
-// 0.97 ms (4.3 GB; 2.5 ms with two reads, double-double tile sums and 32-term
-// replays); n = 20: 0.11 ms (0.38).  A single-read look-back over the tiles
+// about 5 us per binade crossing.  Total probability, complex128, n = 28:
+// 0.86 ms (4.3 GB; 2.5 ms with two reads, double-double tile sums and 32-term
+// replays); n = 20: 0.08 ms (0.38).  A single-read look-back over the tiles
 // measured 1.8 ms and more (its waits drain the loads in flight), the walk in
 // one warp 1.38 ms (a lone warp's step costs as much as the block's).
 #include <algorithm>
@@ -578,7 +578,7 @@ __device__ unsigned walk_records(const SeqRec &r, unsigned l, unsigned cnt, doub
 
 struct ReplayShared {
 	double C;
-	unsigned pos, event, step;
+	unsigned pos, event, step, forgiven;
 	unsigned done;
 	unsigned long long answer;
 	tq::Inc w[kWarps];
@@ -597,16 +597,23 @@ template <class F, bool STOP>
 __device__ void replay_tile(const F &term, unsigned sum, uint64_t base, unsigned cnt, double rnd, double *st, ReplayShared &S) {
 	constexpr bool SIGNED = F::kSigned;
 	const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+	// All 16 loads of a thread before the first use: one at a time, each waiting
+	// for HBM, they were half of the walk (n = 26: 9 us a tile, now 2).
+	typename F::Raw raw[kPer];
+#pragma unroll
+	for(unsigned q = 0; q < kPer; ++q) raw[q] = term.load(base + min(q * kThreads + tid, cnt - 1u));
 #pragma unroll
 	for(unsigned q = 0; q < kPer; ++q) {
 		const unsigned i = q * kThreads + tid;
-		double v[F::kSums] = {};
-		if(i < cnt) term.terms(term.load(base + i), v);
-		st[stage_slot(i)] = F::kSums == 2 && sum == 1 ? v[F::kSums - 1] : v[0];
+		double v[F::kSums];
+		term.terms(raw[q], v);
+		const double x = F::kSums == 2 && sum == 1 ? v[F::kSums - 1] : v[0];
+		st[stage_slot(i)] = i < cnt ? x : 0.0;
 	}
 	if(tid == 0) {
 		S.pos = 0;
 		S.step = kTile;
+		S.forgiven = 0;
 	}
 	__syncthreads();
 	const double *p = st + tid * (kPer + 1);
@@ -719,7 +726,10 @@ __device__ void replay_tile(const F &term, unsigned sum, uint64_t base, unsigned
 			const unsigned to = i0 + k1;
 			S.C = c * inv;
 			S.pos = to;
-			S.step = to - pos;
+			// (A tile's first short step is often a sum that was about to leave anyway:
+			// 256 single additions after it were half of a signed walk, n = 26.)
+			S.step = S.forgiven ? to - pos : kTile;
+			S.forgiven = 1;
 			if(STOP && hit < kPer) {
 				S.C = chit;
 				S.done = 1;
