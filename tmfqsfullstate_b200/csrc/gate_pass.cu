@@ -202,6 +202,27 @@ __device__ __forceinline__ void op_x(Amps<R, RB> &v, bool on) {
 	}
 }
 
+// One phase product of the fast forms.  complex64: each component updated in its
+// own register; from the plain expressions the new values went to registers of
+// their own and were moved back where the operations' paths meet (random circuits
+// of 26 qubits 3.30 ms, now 3.2; complex128 was 8% slower this way, by spills).
+__device__ __forceinline__ void phase_fast(float pr, float pi, float2 &x) {
+	asm volatile(
+		"{\n\t.reg .f32 b, d;\n\t"
+		"mul.rn.f32 b, %3, %1;\n\t"
+		"mul.rn.f32 d, %3, %0;\n\t"
+		"neg.f32 b, b;\n\t"
+		"fma.rn.f32 %0, %2, %0, b;\n\t"
+		"fma.rn.f32 %1, %2, %1, d;\n\t}"
+		: "+f"(x.x), "+f"(x.y)
+		: "f"(pr), "f"(pi));
+}
+__device__ __forceinline__ void phase_fast(double pr, double pi, double2 &x) {
+	const double re = x.x, im = x.y;
+	x.x = fma(pr, re, -(pi * im));
+	x.y = fma(pr, im, pi * re);
+}
+
 // Phase on the registers that have all bits of M.
 template <typename R, unsigned RB, bool EXACT, unsigned M>
 __device__ __forceinline__ void op_cp(Amps<R, RB> &v, R pr, R pi) {
@@ -215,17 +236,16 @@ __device__ __forceinline__ void op_cp(Amps<R, RB> &v, R pr, R pi) {
 #pragma unroll
 	for(unsigned r = 0; r < kRegs; ++r) {
 		if((r & M) != M) continue;
-		R re = v[r].x, im = v[r].y;
 		if constexpr(EXACT) {
 			// Zero amplitudes are skipped (dense_state_backend.cpp:299).
+			R re = v[r].x, im = v[r].y;
 			cmul_ref(pr, pi, re, im);
 			if(least != 0u || nonzero_bits(v[r]) != 0u) {
 				v[r].x = re;
 				v[r].y = im;
 			}
 		} else {
-			v[r].x = fma(pr, re, -(pi * im));
-			v[r].y = fma(pr, im, pi * re);
+			phase_fast(pr, pi, v[r]);
 		}
 	}
 }
