@@ -1029,7 +1029,7 @@ size_t dense_block_extent(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, siz
 // Whether the run of ops starting at ops[i] within 5 qubits is applied as one
 // block sweep.  Gates of one and two qubits do better in the fused passes,
 // which hold gates on 9 to 11 qubits (two-qubit gates on 2^27 complex64
-// amplitudes: about 60 us each there, a block sweep 515 us whatever it holds),
+// amplitudes: about 80 us each there, a block sweep 515 us whatever it holds),
 // unless the block is the whole rest of the batch, or holds many of them.
 bool block_wanted(tmfqs_gpu_state *h, const Planner &p, const tmfqs_op *ops, size_t i, size_t count) {
 	bool has_gate = false;
