@@ -117,3 +117,38 @@ def test_dense_gate_alone_and_at_pass_limits(form):
             g.apply_ops([tq.h(0), tq.gate(u, [3, 9]), tq.gate(u, [4, 4])])
         ref = want(n, a, [O.h(0), O.gate(u, [3, 9])])
         assert np.array_equal(g.export(), ref) if form == "f64" else O.rel_l2(ref, g.export()) <= bound(form, [1, 2])
+
+
+@pytest.mark.parametrize("n", [12, 14, 17])
+@pytest.mark.parametrize("k", [1, 2])
+@pytest.mark.parametrize("where", ["before", "between", "after"])
+@pytest.mark.parametrize("form", ["f64", "f64fast", "c64"])
+def test_gates_beside_rings_of_phases(n, k, where, form):
+    """Layers of small gates around a layer of Hadamards and a ring of controlled phases (the run of phases merges in
+    the fast complex128 form), fused and gate by gate."""
+    rng = np.random.default_rng(n + k)
+
+    def gates(M, seed):
+        return [M.gate(unitary(1 << k, seed + q), list(range(q, q + k))) for q in range(0, n - k + 1, k)]
+
+    def ops(M):
+        t = np.random.default_rng(n).uniform(-3, 3, n)
+        ring = [M.cphase(q, (q + 1) % n, float(t[q])) for q in range(n)]
+        hs = [M.h(q) for q in range(n)]
+        first = {"before": gates(M, 1) + hs + ring, "between": hs + gates(M, 1) + ring, "after": hs + ring + gates(M, 1)}[where]
+        return first + ring + gates(M, 50)
+
+    a = rng.standard_normal(2 << n)
+    a /= np.linalg.norm(a)
+    ref = want(n, a, ops(O))
+    others = len(ops(tq)) - 2 * len(gates(tq, 1))
+    limit = bound(form, [k] * (2 * len(gates(tq, 1)))) + others * (2.0 ** -24 if form == "c64" else 2.0 ** -53)
+    for fusion in (1, 0):
+        with tq.GpuState(tq.FP32 if form == "c64" else tq.FP64) as g:
+            if form == "f64fast":
+                g.set_option(tq.OPT_EXACT, 0)
+            g.set_option(tq.OPT_FUSION, fusion)
+            g.load(n, a)
+            g.apply_ops(ops(tq))
+            got = g.export()
+        assert np.array_equal(got, ref) if form == "f64" else O.rel_l2(ref, got) <= limit

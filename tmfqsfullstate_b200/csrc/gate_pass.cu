@@ -916,7 +916,8 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 
 template <typename R, unsigned RB, bool EXACT>
 bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_prog, size_t &dev_prog_bytes, void *mirror, bool merged) {
-	if(merged && (EXACT || sizeof(R) != 8)) return false;
+	// (the kernel for merged runs has no dense gates: a pass with both takes the one for dense gates)
+	if(merged && (EXACT || sizeof(R) != 8 || !pass.mats.empty())) return false;
 	constexpr unsigned K = tile_bits<R>();
 	GateGeom g;
 	std::vector<GateOp> ops;

@@ -181,8 +181,8 @@ void launch_fused_pass(const LaunchCtx &c, int prec, bool exact, void *a, const 
                        size_t &dev_prog_bytes);
 // Any fused pass on a full tile as register stages (gate_pass.cu); false
 // (nothing launched) when its plan does not fit.  With `merged` (fast complex128
-// form) only a pass nearly all of whose controlled phases merge, and with
-// `mirror` (a state-sized buffer) its result is written there too.
+// form) only a pass without dense gates nearly all of whose controlled phases
+// merge, and with `mirror` (a state-sized buffer) its result is written there too.
 bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const FusedPass &pass, void *&dev_prog,
                       size_t &dev_prog_bytes, void *mirror = nullptr, bool merged = false);
 // The other two kernels of launch_fused_pass (fused.cu): the exact register
