@@ -823,6 +823,9 @@ void run_fused(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_pr
 	g.m = 0;
 	while(g.m < pass.K && pass.lpos[g.m] == g.m) ++g.m;
 	if(g.m == 0 || pass.K > kMaxLocal) fail(TMFQS_ERR_LOGIC, "fused pass: bad local set");
+	// The kernel skips kinds that it does not know (dense gates).
+	for(const FusedOp &op : pass.ops)
+		if(op.kind > kFHTwiddle) fail(TMFQS_ERR_LOGIC, "fused pass: operation kind " + std::to_string(op.kind));
 	for(unsigned i = 0; i < pass.K; ++i) g.lpos[i] = pass.lpos[i];
 	g.ntiles = 1ull << (pass.n - pass.K);
 	g.o_begin = 0;

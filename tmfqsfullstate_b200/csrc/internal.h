@@ -187,7 +187,7 @@ bool launch_gate_pass(const LaunchCtx &c, int prec, bool exact, void *a, const F
                       size_t &dev_prog_bytes, void *mirror = nullptr, bool merged = false);
 // The other two kernels of launch_fused_pass (fused.cu): the exact register
 // stages of Hadamards and their chains (false: nothing launched), and the
-// op-by-op pass, which takes every program.
+// op-by-op pass, which takes every program without dense gates.
 bool launch_fused_stages(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
                          size_t &dev_prog_bytes);
 void launch_fused_ops(const LaunchCtx &c, int prec, void *a, const FusedPass &pass, void *&dev_prog,
