@@ -42,3 +42,32 @@ def test_pass_block_shapes(kind, bits, n, prec):
             if not exact:
                 assert g.stats()["qft_passes"] >= 1
     assert np.linalg.norm(res[1] - res[0]) <= TOL[prec] * np.linalg.norm(res[0])
+
+
+@pytest.mark.parametrize("n", [22, 29])
+def test_factor_rows_of_two_block_passes(n):
+    """Fast complex128 QFTs one of whose two-block passes multiplies by factors of the tile's outer bits (the first at 22
+    qubits, the second at 29): against the exact form, and the same bits in every repetition."""
+    import torch
+
+    gen = torch.Generator(device="cuda:0")
+    gen.manual_seed(n)
+    amps = torch.randn(2 << n, generator=gen, device="cuda:0", dtype=torch.float64)
+    amps /= torch.linalg.vector_norm(amps)
+    ops = tq.qft_ops(n)
+
+    def run(g, exact):
+        g.set_option(tq.OPT_EXACT, exact)
+        g.init_zero(n)
+        g.tensor().copy_(amps)
+        torch.cuda.synchronize()
+        g.apply_ops(ops)
+
+    with tq.GpuState(tq.FP64) as exact, tq.GpuState(tq.FP64) as first, tq.GpuState(tq.FP64) as again:
+        run(exact, 1)
+        run(first, 0)
+        assert first.stats()["qft_passes"] >= 2
+        assert exact.compare(first)["rel_l2"] <= TOL[tq.FP64]
+        for _ in range(20 if n < 25 else 4):
+            run(again, 0)
+            assert first.compare(again)["bitwise_equal"]

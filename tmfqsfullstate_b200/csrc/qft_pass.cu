@@ -321,6 +321,11 @@ __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *b) {
 	asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
+// Plain arrival: what this thread wrote before is seen by those that wait.
+__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
+	asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *b, unsigned parity) {
 	uint32_t ok;
 	asm volatile(
@@ -477,8 +482,13 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 	uint16_t *spst = reinterpret_cast<uint16_t *>(mbar + g.slots);
 
 	if(tid < g.nstages) sst[tid] = g.st[tid];
-	if(tid == 0)
-		for(unsigned k = 0; k < g.slots; ++k) mbar_init(&mbar[k], TM ? 1u : nthr);
+	if(tid == 0) {
+		// ONE: also the threads that write the tile's rows of factors.
+		unsigned arrivals = TM ? 1u : nthr;
+		if(ONE)
+			for(unsigned k = 0; k < g.nstages; ++k) arrivals += g.st[k].ot != kQftNone;
+		for(unsigned k = 0; k < g.slots; ++k) mbar_init(&mbar[k], arrivals);
+	}
 	const uint64_t goff = qft_scatter(g, tid * per16);
 	const unsigned psm = qft_phys(g, tid * per16);
 	const unsigned gstep = nthr * per16;  // shared index step between a thread's granules
@@ -486,7 +496,9 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 
 	// Tile o's amplitudes (16-byte granules at fixed per-thread offsets) and,
 	// from one thread per stage, its row of per-tile factors (the outer bits
-	// of W), computed while the copies are in flight.
+	// of W), computed while the copies are in flight.  In a ring a barrier of
+	// the tile before lies between the row's writes and its use; with one buffer
+	// there is none, and the row's threads arrive on the slot's barrier as well.
 	auto prefetch = [&](uint64_t o, unsigned slot) {
 		if(o < g.ntiles) {
 			const uint64_t base = qft_tile_base(g, o);
@@ -507,9 +519,11 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 				cp_async_mbar_arrive(&mbar[slot]);
 			}
 			const unsigned st = tid >> 5;
-			if((tid & 31u) == 0 && st < g.nstages && sst[st].ot != kQftNone)
+			if((tid & 31u) == 0 && st < g.nstages && sst[st].ot != kQftNone) {
 				stage_factors<V>(base & sst[st].wmask & ~g.localmask, sst[st].bhi, sst[st].d,
 				                 orow + slot * g.ot_stride + sst[st].ot, 1);
+				if(ONE) mbar_arrive(&mbar[slot]);
+			}
 		}
 	};
 	uint64_t o = blockIdx.x;
