@@ -91,6 +91,14 @@ def test_qft_pass_narrow_passes(prec, fq):
     check(n, tq.random_phase(n, 11 * fq), tq.qft_ops(n), prec, fused_qubits=fq)
 
 
+@pytest.mark.parametrize("prec", [tq.FP64, tq.FP32])
+@pytest.mark.parametrize("fq", [1, 2, 3, 4, 5])
+def test_qft_pass_tiles_of_one_warp(prec, fq):
+    """Passes of so few target qubits that a tile has one warp, or is too small for the QFT pass."""
+    n = 19
+    check(n, tq.random_phase(n, 11 * fq), tq.qft_ops(n), prec, expect_qft=fq == 5, fused_qubits=fq)
+
+
 def run_chunks(n, amps, ops, prec, chunk):
     with tq.GpuState(prec) as g:
         g.set_option(tq.OPT_EXACT, 0)

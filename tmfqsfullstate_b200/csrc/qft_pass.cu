@@ -518,11 +518,18 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 				for(unsigned i = 0; i < kGranules; ++i) cp_async16(dst + i * gstep, src + i * g.istride);
 				cp_async_mbar_arrive(&mbar[slot]);
 			}
-			const unsigned st = tid >> 5;
-			if((tid & 31u) == 0 && st < g.nstages && sst[st].ot != kQftNone) {
+			auto row = [&](unsigned st) {
+				if(sst[st].ot == kQftNone) return;
 				stage_factors<V>(base & sst[st].wmask & ~g.localmask, sst[st].bhi, sst[st].d,
 				                 orow + slot * g.ot_stride + sst[st].ot, 1);
 				if(ONE) mbar_arrive(&mbar[slot]);
+			};
+			// (narrow tiles of the ring have fewer warps than stages)
+			if((tid & 31u) == 0) {
+				const unsigned st = tid >> 5;
+				if(st < g.nstages) row(st);
+				if(!ONE)
+					for(unsigned k = st + (nthr >> 5); k < g.nstages; k += nthr >> 5) row(k);
 			}
 		}
 	};
@@ -1005,7 +1012,8 @@ bool run_qft(const LaunchCtx &c, void *a, const FusedPass &pass, const std::vect
 	// 3850, 1934 and 46; complex128 at 29, 27 and 25 4100, 1128 and 230 against 3730,
 	// 1070 and 224.  Passes of two stages have room for the bytes of a tile and
 	// keep the ring (complex128 at 23 qubits 70 us against 72).
-	const bool one = !g.tma && g.nstages >= 3 && smem_for(1) + 1024 <= (size_t)max_optin / 2 &&
+	// (A warp per stage writes the factor rows.)
+	const bool one = !g.tma && g.nstages >= 3 && nthr >= 32 * g.nstages && smem_for(1) + 1024 <= (size_t)max_optin / 2 &&
 	                 g.ntiles >= 4ull * (uint64_t)c.num_sms;
 	if(one) g.slots = 1;
 	const size_t smem = smem_for(g.slots);
