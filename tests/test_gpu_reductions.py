@@ -131,3 +131,36 @@ def test_search_result_at_a_power_of_two(n, marked):
         for r in (0.1, 0.49, 0.7, 1 - 3e-12):
             if r <= cdf[-1]:
                 assert g.sample(r) == int(np.argmax(r <= cdf))
+
+
+@pytest.mark.parametrize("n", [11, 14, 15, 17, 22])
+@pytest.mark.parametrize("kind", ["all", "zeros", "mixed"])
+def test_nan_is_never_lost(n, kind):
+    """All NaN, one NaN in an otherwise zero tile of a basis state, one NaN among terms of both signs: the total and the
+    sums are NaN, and a draw finds its index only among the terms before the NaN."""
+    N = 1 << n
+    rng = np.random.default_rng(n)
+    for at in ((0,) if kind == "all" else (N // 3, N - 7)):
+        for part in (0, 1):
+            a = np.zeros((N, 2))
+            if kind == "all":
+                a[:, part] = np.nan
+            elif kind == "zeros":
+                a[N // 2, 0] = 1.0
+                a[at, part] = np.nan
+            else:
+                a = (1.0 + 2.0 * rng.standard_normal((N, 2))) / np.sqrt(10.0 * N)
+                a[at, part] = np.nan
+            with np.errstate(invalid="ignore"):
+                cdf, sums = np.cumsum(terms(a)), np.cumsum(a, axis=0)[-1]
+                hit = 0.25 <= cdf
+            assert np.isnan(cdf[-1])
+            with tq.GpuState(tq.FP64) as g:
+                g.load(n, a.reshape(-1))
+                assert np.isnan(g.total_probability())
+                assert np.array_equal(g.amplitude_sum(), sums, equal_nan=True)
+                if hit.any():
+                    assert g.sample(0.25) == int(np.argmax(hit))
+                else:
+                    with pytest.raises(tq.RuntimeFailure):
+                        g.sample(0.25)

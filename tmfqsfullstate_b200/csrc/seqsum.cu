@@ -331,8 +331,9 @@ __device__ __forceinline__ void tile_parts(const double *p, int e, bool two, War
 			const double scale = tq::grid_scale(e + k);
 			tq::Inc v = run_increment<SIGNED>(p, scale);
 			// Every run must stay in the binade: it gets at most `mag` away from
-			// where it starts, the middle for signed sums and else the bottom.
-			const bool wide = !(w.mag * (SIGNED ? 2.0 : 1.0) * scale < kBinade);
+			// where it starts, the middle for signed sums and else the bottom.  (`mag` of
+			// mixed signs knows nothing of a NaN; the sum does.)
+			const bool wide = !(w.mag * (SIGNED ? 2.0 : 1.0) * scale < kBinade) || w.s != w.s;
 			if(__all_sync(FULL, v.i0 == v.i1)) {
 #pragma unroll
 				for(unsigned d = 16; d > 0; d >>= 1) v.i0 += __shfl_xor_sync(FULL, v.i0, d);
@@ -372,7 +373,7 @@ __device__ __forceinline__ SeqRec parts_join(const WarpPart *parts, int e, bool 
 		}
 	}
 	if(!SIGNED) r.mx = r.s;
-	if(mag == 0.0) return r;
+	if(mag == 0.0 && r.s == 0.0) return r;  // (fmax passes over a NaN)
 	r.e = e;
 	r.ok = signs | (e == tq::kDirty ? 0u : (two ? kHasE | kHasE1 : kHasE) & ~wide);
 	for(unsigned k = 0; k < 2; ++k) {
@@ -621,7 +622,7 @@ __device__ void replay_tile(const F &term, unsigned sum, uint64_t base, unsigned
 	for(;;) {
 		const double C = S.C;
 		const unsigned pos = S.pos, step = S.step;
-		if(pos >= cnt || S.done) break;
+		if(pos >= cnt || S.done || C != C) break;
 		__syncthreads();
 		if(tid == 0) S.event = cnt;
 		__syncthreads();
@@ -763,7 +764,7 @@ __device__ void walk_block(const F &term, unsigned sum, uint64_t N, const SeqTab
 		if(tid < 32) {
 			unsigned tile = T.ntiles;
 			double C = S.C;
-			if(S.done) {
+			if(S.done || C != C) {  // (no term changes a NaN, and no draw reaches it)
 			} else if(direct) {
 				tile = t++;
 			} else {
