@@ -60,8 +60,8 @@ constexpr unsigned kSpinLimit = 1u << 20;
 
 // Effect of a run of terms on the running sum (tile or group): grid increments
 // for binades e and e + 1, and for signed sums the run's sum and the extremes
-// of its prefix sums.
-struct SeqRec {
+// of its prefix sums.  (Copied in 16-byte words.)
+struct alignas(16) SeqRec {
 	int e;        // tq::kIdentity: all terms zero
 	unsigned ok;  // kHasE, kHasE1: the increments that are known; kUp, kDown: no term is negative / positive
 	long long i0[2], i1[2];
@@ -167,6 +167,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ __forceinline__ unsigned stage_slot(unsigned i) { return i + i / kPer; }
 
 __device__ __forceinline__ SeqRec load_rec(const SeqRec *p) {
+	static_assert(alignof(SeqRec) >= alignof(int4) && sizeof(SeqRec) % sizeof(int4) == 0, "records are copied as int4");
 	SeqRec r;
 	const int4 *src = reinterpret_cast<const int4 *>(p);
 	int4 *dst = reinterpret_cast<int4 *>(&r);
