@@ -107,6 +107,22 @@ def test_more_operations_than_one_plan_holds(prec):
         assert O.rel_l2(ref, got) <= 400 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("n", [13, 14, 16])
+@pytest.mark.parametrize("form,size", [("c64", 1e30), ("c64", 1e-30), ("f64fast", 1e290)])
+def test_many_hadamards_far_from_norm_one(n, form, size):
+    """220 operations, mostly Hadamards, on values next to the ends of the range: the outstanding powers of sqrt(2) stay small."""
+    ops = circuit(n, 220, n, "hhhhhhhhc", list(range(8)))
+    a = inputs("random", n, 7) * size
+    with tq.GpuState(tq.FP32 if form == "c64" else tq.FP64) as g:
+        if form == "f64fast":
+            g.set_option(tq.OPT_EXACT, 0)
+        g.load(n, a)
+        g.apply_ops(build(ops, tq))
+        got = g.export()
+    ref = want(n, a / size, ops)
+    assert O.rel_l2(ref, got / size) <= 220 * (2.0 ** -24 if form == "c64" else 2.0 ** -53)
+
+
 def rings(n, layers, seed, extra):
     """Hadamard layers with rings of phases, and `extra` random phases after each (pairs in every position)."""
     rng = np.random.default_rng(seed)

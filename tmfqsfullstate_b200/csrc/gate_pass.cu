@@ -15,7 +15,8 @@
 // Exact form: the IEEE operations of the per-gate path in circuit order for each
 // amplitude (dense_state_backend.cpp:255-319), zero pairs and zero amplitudes
 // skipped as there, so the result is bit-identical.  Fast forms: butterflies
-// without their 1/sqrt(2), which is applied once as a power at the end.
+// without their 1/sqrt(2), which is applied once as a power at the end; on the way
+// the powers of two in it after every kMaxDeferred butterflies, exactly.
 //
 // Bound: HBM (one read and one write per pass) and, behind it, instruction issue:
 // about 60 instructions per operation and 16 amplitudes, at half the issue rate
@@ -44,6 +45,10 @@ constexpr unsigned kMaxRB = 5;
 constexpr unsigned kMaxK = 13;
 constexpr unsigned kMaxStages = 64;
 constexpr unsigned kMaxOps = 240;
+// Fast forms: the Hadamards whose 1/sqrt(2) is outstanding at one time, as in the
+// radix passes on a tile.  (240 of them would be 2^120: a complex64 register that
+// is not normalised overflowed from values of 10^3 on.)
+constexpr unsigned kMaxDeferred = 12;
 
 // Tiles of 64 KiB.
 template <typename R>
@@ -78,7 +83,9 @@ constexpr unsigned line_bits() {
 // fast forms always the higher one).
 // kCodeDiag: a merged run of controlled phases, tmask the register bits with a
 // factor, rval its number, omask the thread bits with a factor per tile.
-constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeFlip = 62, kCodeU1 = 63, kCodeU2 = 68, kCodeDiag = 100;
+// kCodeScale (a phase on three register bits, which there is not): all
+// amplitudes times cr.
+constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeScale = kCodeCP + 7, kCodeFlip = 62, kCodeU1 = 63, kCodeU2 = 68, kCodeDiag = 100;
 
 // Merged runs of controlled phases (fast complex128 form).  In a run the phases commute, so
 // those without two register bits collect into one factor per thread and one
@@ -121,7 +128,7 @@ struct GateGeom {
 	double inv, scale;  // 1/sqrt(2); fast forms: the pass's power of it
 	uint64_t outer;     // mask of the index bits outside the tile
 	uint8_t lpos[kMaxK], opos[kMaxK];  // index bit of a tile bit when loaded and when stored
-	uint8_t first[kMaxStages], count[kMaxStages];
+	uint16_t first[kMaxStages], count[kMaxStages];
 	uint8_t rbit[kMaxStages][kMaxRB];        // tile bit of register bit i
 	uint8_t tbit[kMaxStages][kMaxTB];  // tile bit of thread index bit k
 };
@@ -473,6 +480,15 @@ __device__ __forceinline__ void run_op(const OpS<R> &op, Amps<R, RB> &v, const G
 		return;
 		TQB_CP(0) TQB_CP(1) TQB_CP(2) TQB_CP(3) TQB_CP(4) TQB_CP(5) TQB_CP(6) TQB_CP(8) TQB_CP(9) TQB_CP(10) TQB_CP(12)
 		TQB_CP(16) TQB_CP(17) TQB_CP(18) TQB_CP(20) TQB_CP(24)
+	case kCodeScale:
+		if constexpr(!EXACT) {
+#pragma unroll
+			for(unsigned r = 0; r < Amps<R, RB>::kRegs; ++r) {
+				v[r].x *= pr;
+				v[r].y *= pr;
+			}
+		}
+		return;
 		default: return;
 #undef TQB_H
 #undef TQB_X
@@ -771,6 +787,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 	terms.clear();
 	loose = 0;
 	mats = pass.mats;
+	unsigned deferred = 0, halvings = 0;  // Hadamards since the last kCodeScale, and the powers of two applied by those
 	for(unsigned st = 0; st < g.nstages; ++st) {
 		const bool in = st == 0, outs = st + 1 == g.nstages;
 		const uint32_t fixed = (in ? keep_in : 0u) | (outs ? keep_out : 0u);
@@ -814,7 +831,7 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 		while(!rest.empty()) take(rest.front());
 		for(unsigned i = 0; i < RB; ++i) g.rbit[st][i] = (uint8_t)rb[i];
 		for(unsigned k = 0; k < tb.size(); ++k) g.tbit[st][k] = (uint8_t)tb[k];
-		g.first[st] = (uint8_t)out.size();
+		g.first[st] = (uint16_t)out.size();
 		for(unsigned pos = 0; pos < of[st].size(); ++pos) {
 			const unsigned k = of[st][pos];
 			const PlanOp &q = ops[k];
@@ -904,13 +921,22 @@ bool plan_gates(const FusedPass &pass, unsigned K, unsigned RB, unsigned line, b
 					break;
 			}
 			out.push_back(o);
+			if(!exact && q.kind == PlanOp::kH && ++deferred == kMaxDeferred) {
+				GateOp x{};
+				x.code = kCodeScale;
+				x.cr = std::ldexp(1.0, -(int)(kMaxDeferred / 2));
+				out.push_back(x);
+				deferred = 0;
+				halvings += kMaxDeferred / 2;
+			}
 		}
-		g.count[st] = (uint8_t)(out.size() - g.first[st]);
+		g.count[st] = (uint16_t)(out.size() - g.first[st]);
 	}
 	g.nops = (unsigned)out.size();
 	g.nterms = (unsigned)terms.size();
 	g.nmat = (unsigned)(pass.mats.size() / 2);
-	g.scale = std::pow(g.inv, (double)nh);  // of the reference's 1/sqrt(2), rounded as it is: the difference adds up
+	// The power of the reference's 1/sqrt(2), rounded as it is (the difference adds up).
+	g.scale = std::ldexp(std::pow(g.inv, (double)nh), (int)halvings);
 	return true;
 }
 
