@@ -518,18 +518,11 @@ __global__ void __launch_bounds__(qft_max_threads(sizeof(typename Vec2<R>::type)
 				for(unsigned i = 0; i < kGranules; ++i) cp_async16(dst + i * gstep, src + i * g.istride);
 				cp_async_mbar_arrive(&mbar[slot]);
 			}
-			auto row = [&](unsigned st) {
-				if(sst[st].ot == kQftNone) return;
+			const unsigned st = tid >> 5;
+			if((tid & 31u) == 0 && st < g.nstages && sst[st].ot != kQftNone) {
 				stage_factors<V>(base & sst[st].wmask & ~g.localmask, sst[st].bhi, sst[st].d,
 				                 orow + slot * g.ot_stride + sst[st].ot, 1);
 				if(ONE) mbar_arrive(&mbar[slot]);
-			};
-			// (narrow tiles of the ring have fewer warps than stages)
-			if((tid & 31u) == 0) {
-				const unsigned st = tid >> 5;
-				if(st < g.nstages) row(st);
-				if(!ONE)
-					for(unsigned k = st + (nthr >> 5); k < g.nstages; k += nthr >> 5) row(k);
 			}
 		}
 	};
@@ -802,6 +795,9 @@ bool plan_qft(const FusedPass &pass, const std::vector<unsigned> &hb, unsigned r
 			S.direct = ok;
 		}
 	}
+	// A stage's row of factors is written by the warp of its number: tiles with
+	// fewer warps than stages (narrow passes) run as radix passes.
+	if(ocol && (32u * nst) > (1u << (K - RB))) return false;
 	g.nfrows = nfrows;
 	g.ot_stride = ocol;
 
@@ -1012,8 +1008,7 @@ bool run_qft(const LaunchCtx &c, void *a, const FusedPass &pass, const std::vect
 	// 3850, 1934 and 46; complex128 at 29, 27 and 25 4100, 1128 and 230 against 3730,
 	// 1070 and 224.  Passes of two stages have room for the bytes of a tile and
 	// keep the ring (complex128 at 23 qubits 70 us against 72).
-	// (A warp per stage writes the factor rows.)
-	const bool one = !g.tma && g.nstages >= 3 && nthr >= 32 * g.nstages && smem_for(1) + 1024 <= (size_t)max_optin / 2 &&
+	const bool one = !g.tma && g.nstages >= 3 && smem_for(1) + 1024 <= (size_t)max_optin / 2 &&
 	                 g.ntiles >= 4ull * (uint64_t)c.num_sms;
 	if(one) g.slots = 1;
 	const size_t smem = smem_for(g.slots);
