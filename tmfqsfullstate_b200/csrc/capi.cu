@@ -1000,62 +1000,91 @@ bool op_as_matrix(const tmfqs_op &op, std::vector<unsigned> &qs, std::vector<std
 // FP64, which rounds differently from the reference's gate-by-gate products.
 bool block_fusion(const tmfqs_gpu_state *h) { return h->precision == TMFQS_FP32 || !h->opt_exact; }
 
-// The run of ops starting at ops[i] that acts within 5 qubits and that a
-// block can take: its end (exclusive), and whether it holds a dense gate
-// (MatrixGate) -- runs without one are left to the fused passes.
-size_t dense_block_extent(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, size_t count, bool &has_gate) {
-	std::vector<unsigned> Q;
-	has_gate = false;
-	size_t j = i;
-	for(; j < count; ++j) {
-		std::vector<unsigned> qs;
-		std::vector<std::complex<double>> g;
-		try {
-			validate_op(h, ops[j]);
-		} catch(const tqb::Error &) {
-			break;  // the ops before an invalid one are applied, then it is reported
-		}
-		if(!op_as_matrix(ops[j], qs, g)) break;
-		std::vector<unsigned> U = Q;
-		for(unsigned q : qs)
-			if(std::find(U.begin(), U.end(), q) == U.end()) U.push_back(q);
-		if(U.size() > 5) break;
-		Q = U;
-		has_gate = has_gate || ops[j].kind == TMFQS_OP_GATE;
+// The qubits of an op that a block can take (false: it cannot).
+bool block_qubits(const tmfqs_op &op, unsigned (&qs)[5], unsigned &k) {
+	switch(op.kind) {
+		case TMFQS_OP_H:
+		case TMFQS_OP_X: k = 1; break;
+		case TMFQS_OP_CNOT:
+		case TMFQS_OP_CPHASE:
+		case TMFQS_OP_SWAP: k = 2; break;
+		case TMFQS_OP_GATE:
+			k = op.k;
+			if(k == 0 || k > 5) return false;
+			std::copy(op.qubits, op.qubits + k, qs);
+			return true;
+		default: return false;
 	}
-	return j;
+	qs[0] = op.q0;
+	qs[1] = op.q1;
+	return true;
 }
 
-// Whether the run of ops starting at ops[i] within 5 qubits is applied as one
+// The run of ops starting at some op that acts within 5 qubits and that a block
+// can take: its end (exclusive), and the dense gates (MatrixGates) in it -- runs
+// without one are left to the fused passes.  From one start to a later one only
+// the ops between them leave the run and only ops after its end join it, so a
+// batch's runs are found in one walk over it.
+struct BlockRun {
+	tmfqs_gpu_state *h;
+	const tmfqs_op *ops;
+	size_t count;
+	size_t begin = 0, end = 0;
+	unsigned gates = 0, wide = 0;  // dense gates, and those of more than two qubits
+	unsigned distinct = 0;
+	unsigned uses[64] = {};  // ops of the run on each qubit
+
+	BlockRun(tmfqs_gpu_state *hh, const tmfqs_op *o, size_t c) : h(hh), ops(o), count(c) {}
+
+	void start_at(size_t i) {
+		unsigned qs[5], k = 0;
+		for(; begin < i && begin < end; ++begin) {
+			block_qubits(ops[begin], qs, k);
+			for(unsigned a = 0; a < k; ++a) distinct -= --uses[qs[a]] == 0;
+			if(ops[begin].kind == TMFQS_OP_GATE) {
+				--gates;
+				wide -= k > 2;
+			}
+		}
+		begin = i;
+		end = std::max(end, i);
+		for(; end < count; ++end) {
+			try {
+				validate_op(h, ops[end]);
+			} catch(const tqb::Error &) {
+				break;  // the ops before an invalid one are applied, then it is reported
+			}
+			if(!block_qubits(ops[end], qs, k)) break;
+			unsigned fresh = 0;
+			for(unsigned a = 0; a < k; ++a) fresh += uses[qs[a]] == 0;
+			if(distinct + fresh > 5) break;
+			distinct += fresh;
+			for(unsigned a = 0; a < k; ++a) ++uses[qs[a]];
+			if(ops[end].kind == TMFQS_OP_GATE) {
+				++gates;
+				wide += k > 2;
+			}
+		}
+	}
+};
+
+// Whether a run of ops within 5 qubits is applied as one
 // block sweep.  Gates of one and two qubits do better in the fused passes,
 // which hold gates on 9 to 11 qubits (two-qubit gates on 2^27 complex64
 // amplitudes: about 80 us each there, a block sweep 515 us whatever it holds),
 // unless the block is the whole rest of the batch, or holds many of them.
-bool block_wanted(tmfqs_gpu_state *h, const Planner &p, const tmfqs_op *ops, size_t i, size_t count) {
-	bool has_gate = false;
-	const size_t jend = dense_block_extent(h, ops, i, count, has_gate);
-	if(!has_gate || jend - i < 2) return false;
+bool block_wanted(const Planner &p, const BlockRun &run) {
+	if(!run.gates || run.end - run.begin < 2) return false;
 	if(!p.takes_dense(2)) return true;
-	unsigned gates = 0, wide = 0;
-	for(size_t j = i; j < jend; ++j)
-		if(ops[j].kind == TMFQS_OP_GATE) {
-			++gates;
-			wide += ops[j].k > 2;
-		}
-	return wide || gates >= 8 || (p.pending.empty() && jend == count);
+	return run.wide || run.gates >= 8 || (p.pending.empty() && run.end == run.count);
 }
 
-// Starting at ops[i], the longest run of ops acting within 5 qubits (holding
-// a dense gate), multiplied in FP64 into one block matrix and applied in one
-// sweep: a tensor-core gate for complex64 (padded to 4 qubits), the CUDA-core
-// block kernel for the fast complex128 form.  Returns the number of ops
-// consumed (0: no block).
-size_t run_dense_block(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, size_t count) {
+// The ops [i, jend) (a BlockRun with a dense gate), multiplied in FP64 into one
+// block matrix and applied in one sweep: a tensor-core gate for complex64
+// (padded to 4 qubits), the CUDA-core block kernel for the fast complex128 form.
+// Returns the number of ops consumed (0: no block).
+size_t run_dense_block(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, size_t jend) {
 	typedef std::complex<double> C;
-	if(!block_fusion(h)) return 0;
-	bool has_gate = false;
-	const size_t jend = dense_block_extent(h, ops, i, count, has_gate);
-	if(!has_gate || jend - i < 2) return 0;
 	std::vector<unsigned> Q;  // block qubits, block order (first = most significant)
 	std::vector<std::pair<std::vector<unsigned>, std::vector<C>>> parts;
 	size_t j = i;
@@ -1063,7 +1092,6 @@ size_t run_dense_block(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t i, size_t
 		std::vector<unsigned> qs;
 		std::vector<C> g;
 		op_as_matrix(ops[j], qs, g);
-		validate_op(h, ops[j]);
 		for(unsigned q : qs)
 			if(std::find(Q.begin(), Q.end(), q) == Q.end()) Q.push_back(q);
 		parts.push_back({qs, g});
@@ -1168,6 +1196,7 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 	p.base = ops;
 	bool blocks = false;
 	for(size_t j = 0; j < count && !blocks; ++j) blocks = block_fusion(h) && ops[j].kind == TMFQS_OP_GATE;
+	BlockRun block(h, ops, count);
 	size_t i = 0;
 	try {
 		while(i < count) {
@@ -1202,11 +1231,12 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 			}
 			// A dense gate, or gates that lead into one, and the ops after it
 			// that stay within 5 qubits: one block sweep.
-			if(blocks && block_wanted(h, p, ops, i, count)) {
+			if(blocks) block.start_at(i);
+			if(blocks && block_wanted(p, block)) {
 				p.flush();
 				h->cur_first = i;
 				h->cur_count = 1;
-				const size_t used = run_dense_block(h, ops, i, count);
+				const size_t used = run_dense_block(h, ops, i, block.end);
 				if(used) {
 					i += used;
 					continue;
