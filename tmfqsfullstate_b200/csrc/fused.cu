@@ -875,7 +875,7 @@ void run_fused(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_pr
 	if(!maps.empty()) std::memcpy(host.data() + map_off, maps.data(), maps.size() * sizeof(ChainMap));
 	upload_async(c, dev_prog, host.data(), need, "fused program upload");
 	const size_t smem = (sizeof(typename Vec2<R>::type) << pass.K) + (sizeof(uint64_t) << (pass.K - g.m));
-	check_cuda(cudaFuncSetAttribute(k_fused<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "fused smem");
+	allow_dynamic_smem(k_fused<R>, "fused smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<R>, kFusedThreads, smem), "fused occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));
@@ -969,7 +969,7 @@ void run_perm(const LaunchCtx &c, void *a, unsigned n, const std::vector<std::pa
 		fail(TMFQS_ERR_LOGIC, "bit permutation: tile larger than the per-thread granule maps");
 	const size_t smem = 4 * (sizeof(typename Vec2<R>::type) << g.K) + (sizeof(uint64_t) << (g.K - g.m)) +
 	                    sizeof(uint64_t) * kPermChunks * 64 * 3 + 4 * H * sizeof(uint16_t);
-	check_cuda(cudaFuncSetAttribute(k_bit_perm<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "perm smem");
+	allow_dynamic_smem(k_bit_perm<R>, "perm smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bit_perm<R>, kPermThreads, smem), "perm occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles, (uint64_t)c.num_sms * std::max(1, per_sm));
@@ -1613,7 +1613,7 @@ bool run_fused_stages(const LaunchCtx &c, void *a, const FusedPass &pass, void *
 	unsigned char *dp = static_cast<unsigned char *>(dev_prog);
 	const size_t smem = stage_smem_layout(sizeof(typename Vec2<R>::type), g.m, g.nops, g.nentries, g.nstages).total;
 	auto kern = g.narrow ? k_fused_stages<R, true> : k_fused_stages<R, false>;
-	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "stage smem");
+	allow_dynamic_smem(kern, "stage smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStThreads, smem), "stage occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));

@@ -979,7 +979,7 @@ bool run_gate_pass(const LaunchCtx &c, void *a, const FusedPass &pass, void *&de
 	auto kern = mats.empty() ? k_gate_pass<R, RB, EXACT, kPlain> : k_gate_pass<R, RB, EXACT, kDense>;
 	if constexpr(!EXACT && sizeof(R) == 8 && RB != small_bits<R>())
 		if(merged) kern = k_gate_pass<R, RB, EXACT, kMerged>;
-	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gate pass smem");
+	allow_dynamic_smem(kern, "gate pass smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem), "gate pass occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));

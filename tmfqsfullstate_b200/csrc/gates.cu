@@ -496,7 +496,7 @@ void run_gate_dense(const LaunchCtx &c, void *a, unsigned n, unsigned k, const d
 	typedef typename Vec2<R>::type V;
 	const size_t smem = sizeof(V) * ((1u << kDenseBits) + kDenseChunk) + sizeof(uint16_t) * (1u << k);
 	auto kern = k_gate_dense<R, EXACT>;
-	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "dense gate smem");
+	allow_dynamic_smem(kern, "dense gate smem");
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem), "dense gate occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles, (uint64_t)c.num_sms * std::max(1, per_sm));
@@ -530,7 +530,7 @@ void dispatch_gate(const LaunchCtx &c, bool exact, void *a, unsigned n, unsigned
 		k_gate_small<R><<<grid_for(c, nblocks), kThreads, 0, c.stream>>>(p, nblocks, g, m);
 	} else {
 		const size_t sm = 2ull * (1ull << k) * sizeof(typename Vec2<R>::type);
-		if(sm > 48 * 1024) check_cuda(cudaFuncSetAttribute(k_gate_block<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), "gate smem");
+		if(sm > 48 * 1024) allow_dynamic_smem(k_gate_block<R>, "gate smem");
 		const unsigned threads = k <= 6 ? 64 : 256;
 		const uint64_t blocks = std::min<uint64_t>(nblocks, (uint64_t)c.num_sms * 16u);
 		k_gate_block<R><<<(unsigned)blocks, threads, sm, c.stream>>>(p, nblocks, g, m);

@@ -1021,7 +1021,7 @@ bool run_qft(const LaunchCtx &c, void *a, const FusedPass &pass, const std::vect
 	if constexpr(sizeof(V) == 8) {  // tensor-map tiles: complex64 only
 		if(g.tma) kern = k_qft_pass<R, RB, true, false>;
 	}
-	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "qft smem");
+	allow_dynamic_smem(kern, "qft smem");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles, (uint64_t)c.num_sms * (one ? 2u : 1u));
 	kern<<<(unsigned)grid, nthr, smem, c.stream>>>(static_cast<V *>(a), g, tmap, c.err);
 	check_cuda(cudaGetLastError(), "qft pass");
