@@ -66,6 +66,18 @@ def test_wide_gates(n, k, where):
         assert O.rel_l2(ref, apply("c64", n, a, [tq.gate(u, q)])) <= bound("c64", [k])
 
 
+@pytest.mark.parametrize("n,k", [(14, 3), (15, 3), (16, 3), (15, 6), (16, 7), (15, 8), (16, 8), (16, 9), (17, 9), (17, 10), (18, 10)])
+def test_wide_gates_where_the_kernel_changes(n, k):
+    """Registers on both sides of the line between one CTA per block and the tiled kernel."""
+    for where in ("low", "any"):
+        u, q = unitary(1 << k, k), targets(n, k, where)
+        for a in (state(n, n + k), state(n, k, sparse=True)):
+            ref = want(n, a, [O.gate(u, q)])
+            assert np.array_equal(apply("f64", n, a, [tq.gate(u, q)]), ref)
+            for form in ("f64fast", "c64"):
+                assert O.rel_l2(ref, apply(form, n, a, [tq.gate(u, q)])) <= bound(form, [k])
+
+
 def mixed(n, count, seed, dense_only=False):
     rng = np.random.default_rng(seed)
     ours, theirs, ks = [], [], []

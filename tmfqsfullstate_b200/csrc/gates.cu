@@ -308,9 +308,10 @@ __global__ void k_gate_small(typename Vec2<R>::type *a, uint64_t nblocks, GateGe
 	}
 }
 
-// k == 0, and 3 <= k <= 10 on states smaller than a tile of k_gate_dense: one
-// CTA per block; amplitudes staged in shared memory.
-template <typename R>
+// k == 0, and 3 <= k <= 10 on states of at most a few tiles of k_gate_dense
+// (gate_by_blocks): one CTA per block; amplitudes staged in shared memory.  Without
+// EXACT the products of k_gate_dense, in the same order.
+template <typename R, bool EXACT>
 __global__ void k_gate_block(typename Vec2<R>::type *a, uint64_t nblocks, GateGeom g, const double *m) {
 	extern __shared__ unsigned char smem_raw[];
 	typedef typename Vec2<R>::type V;
@@ -331,8 +332,13 @@ __global__ void k_gate_block(typename Vec2<R>::type *a, uint64_t nblocks, GateGe
 			const double *row = m + 2ull * r * bs;
 			for(unsigned col = 0; col < bs; ++col) {
 				const R gr = (R)row[2 * col], gi = (R)row[2 * col + 1];
-				nr = radd(nr, rsub(rmul(gr, loc[col].x), rmul(gi, loc[col].y)));
-				ni = radd(ni, radd(rmul(gr, loc[col].y), rmul(gi, loc[col].x)));
+				if constexpr(EXACT) {
+					nr = radd(nr, rsub(rmul(gr, loc[col].x), rmul(gi, loc[col].y)));
+					ni = radd(ni, radd(rmul(gr, loc[col].y), rmul(gi, loc[col].x)));
+				} else {
+					nr = fma(-gi, loc[col].y, fma(gr, loc[col].x, nr));
+					ni = fma(gi, loc[col].x, fma(gr, loc[col].y, ni));
+				}
 			}
 			out[r].x = nr;
 			out[r].y = ni;
@@ -343,7 +349,7 @@ __global__ void k_gate_block(typename Vec2<R>::type *a, uint64_t nblocks, GateGe
 	}
 }
 
-// Dense gates with 3 <= k <= 10 on states of at least one tile: each block
+// Dense gates with 3 <= k <= 10 on larger states (gate_by_blocks): each block
 // reads a tile of 2^12 amplitudes (the targets and the lowest other bits) into
 // shared memory, every thread forms 4 rows x 4 groups of outputs in registers
 // while the matrix passes through shared memory in chunks of columns, and the
@@ -503,9 +509,23 @@ void run_gate_dense(const LaunchCtx &c, void *a, unsigned n, unsigned k, const d
 	kern<<<(unsigned)grid, kThreads, smem, c.stream>>>(static_cast<V *>(a), g, reinterpret_cast<const double2 *>(m));
 }
 
+// Whether a gate on k >= 3 qubits runs as one CTA per block although the state has
+// whole tiles: with few of either, the blocks spread over more SMs.  Calls of
+// exact complex128 gates, block / tile kernel: k = 3 36 / 41 us at 15 qubits, 41 / 42
+// at 16, 49 / 41 at 17; k = 6 57 / 68, 70 / 69, 103 / 69; k = 8 264 / 341, 333 / 343,
+// 486 / 340; k = 9 1082 / 1212 at 16, 1358 / 1216 at 17; k = 10 4098 / 4736 at 17, 5258 /
+// 4769 at 18.  Fast complex128 likewise (k = 6 56 / 57 at 15); complex64 one qubit
+// earlier (k = 7 79 / 88 at 14, 95 / 88 at 15), k = 10 never (3865 / 3818 at 12).
+template <typename R>
+bool gate_by_blocks(const LaunchCtx &c, unsigned n, unsigned k) {
+	if(n < kDenseBits) return true;
+	if(sizeof(R) == 4 && k == 10) return false;
+	return n <= (sizeof(R) == 8 ? 15u : 14u) || (1ull << (n - k)) <= (uint64_t)c.num_sms;
+}
+
 template <typename R>
 void dispatch_gate(const LaunchCtx &c, bool exact, void *a, unsigned n, unsigned k, const double *m, const unsigned *tpos) {
-	if(k >= 3 && n >= kDenseBits) {
+	if(k >= 3 && !gate_by_blocks<R>(c, n, k)) {
 		if constexpr(sizeof(R) == 8) {
 			if(exact) run_gate_dense<R, true>(c, a, n, k, m, tpos);
 			else run_gate_dense<R, false>(c, a, n, k, m, tpos);
@@ -530,10 +550,12 @@ void dispatch_gate(const LaunchCtx &c, bool exact, void *a, unsigned n, unsigned
 		k_gate_small<R><<<grid_for(c, nblocks), kThreads, 0, c.stream>>>(p, nblocks, g, m);
 	} else {
 		const size_t sm = 2ull * (1ull << k) * sizeof(typename Vec2<R>::type);
-		if(sm > 48 * 1024) allow_dynamic_smem(k_gate_block<R>, "gate smem");
+		// (k == 0 and states smaller than a tile: the reference's products in every form)
+		auto kern = k == 0 || n < kDenseBits || (exact && sizeof(R) == 8) ? k_gate_block<R, true> : k_gate_block<R, false>;
+		if(sm > 48 * 1024) allow_dynamic_smem(kern, "gate smem");
 		const unsigned threads = k <= 6 ? 64 : 256;
 		const uint64_t blocks = std::min<uint64_t>(nblocks, (uint64_t)c.num_sms * 16u);
-		k_gate_block<R><<<(unsigned)blocks, threads, sm, c.stream>>>(p, nblocks, g, m);
+		kern<<<(unsigned)blocks, threads, sm, c.stream>>>(p, nblocks, g, m);
 	}
 	after_launch(c, "gate");
 }
