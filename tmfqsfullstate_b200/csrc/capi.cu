@@ -433,6 +433,37 @@ struct Planner {
 		return extra + std::min(mlow, h->n) <= K;
 	}
 
+	// Whether the pass holds only what the fast forms' QFT and radix passes take.
+	bool radix_ops() const {
+		bool hadamard = false;
+		for(const tqb::FusedOp &f : pass.ops) {
+			if(f.kind != tqb::kFH && f.kind != tqb::kFHChain && f.kind != tqb::kFCP) return false;
+			hadamard = hadamard || f.kind != tqb::kFCP;
+		}
+		return hadamard && h->opt_radix;
+	}
+
+	// Whether a run of disjoint swaps (bits m) goes into the fused passes.  A swap
+	// of tile bits is free in a pass of a full tile (it relabels them), a
+	// permutation is a sweep of its own: short runs go into the passes, and so do
+	// longer ones whose bits the current pass holds anyway (exact form; the fast
+	// forms' QFT pass takes no swaps).  Narrower tiles swap in shared memory, which
+	// still saves a launch (QFT of 11 qubits 72 us against 76), but
+	//  - of a part of the register (few target qubits per pass asked for) only
+	//    where the run does not end the pass: circuits of 21 and 23 qubits in passes
+	//    of 3 take 1.73 and 5.67 ms, in the pass whatever it holds 1.97 and 6.98, as
+	//    permutations 1.74 and 5.70 (22 qubits in passes of 7: 0.45, 0.45, 0.54);
+	//  - not as a whole batch (18 us against 22), and not at the end of one after what
+	//    the fast forms' QFT and radix passes take (7 of 12 qubits complex64: 28 us
+	//    against 52; from 10 qubits on, at 8 27 against 24).
+	bool takes_swaps(size_t run, uint64_t m, bool ends) const {
+		if(run < 2) return true;
+		if(K == Kfull) return run < 4 || (exact_form() && fits(m));
+		if(run >= 4 && !exact_form()) return false;
+		if(K < h->n) return fits(m);
+		return !ends || !(pending.empty() || (!exact_form() && h->n >= 10 && radix_ops()));
+	}
+
 	unsigned local_index(unsigned bit) const {
 		for(unsigned i = 0; i < pass.K; ++i)
 			if(pass.lpos[i] == bit) return i;
@@ -1204,17 +1235,12 @@ bool apply_ops_body(tmfqs_gpu_state *h, const tmfqs_op *ops, size_t count, bool 
 			validate_op(h, op);
 			if(op.kind == TMFQS_OP_SWAP) {
 				const size_t run = swap_run(ops, i, count);
-				// A swap of tile bits is free in a fused pass (it relabels them), the
-				// permutation a sweep of its own: short runs go into the passes, and so
-				// do longer ones whose bits the current pass holds anyway (exact form;
-				// the fast forms' QFT pass takes no swaps).
 				uint64_t m = 0;
 				for(size_t j = i; j < i + run; ++j) {
 					validate_op(h, ops[j]);
 					m |= (1ull << bit_of(h, ops[j].q0)) | (1ull << bit_of(h, ops[j].q1));
 				}
-				const bool in_pass = run < 4 || (p.exact_form() && p.fits(m));
-				if(!in_pass) {
+				if(!p.takes_swaps(run, m, i + run == count)) {
 					p.flush();
 					std::vector<std::pair<unsigned, unsigned>> pairs;
 					for(size_t j = i; j < i + run; ++j) pairs.push_back({bit_of(h, ops[j].q0), bit_of(h, ops[j].q1)});
