@@ -164,3 +164,28 @@ def test_nan_is_never_lost(n, kind):
                 else:
                     with pytest.raises(tq.RuntimeFailure):
                         g.sample(0.25)
+
+
+@pytest.mark.parametrize("n", [9, 12, 13, 15, 18])
+@pytest.mark.parametrize("share", [0.002, 0.02, 0.2, 0.5])
+def test_terms_added_one_by_one(n, share):
+    """Sums that the steps over whole tiles do not carry: signed ones that hover around zero with a few or many terms that
+    are not zero (windows of 32 with none, some and all of them), totals whose binade doubles every 4 to 40 terms or that
+    stay below the normal range, and draws that end inside such a run."""
+    N = 1 << n
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((N, 2)) * (rng.random((N, 2)) < share)
+    a[rng.random((N, 2)) < 0.01] = -0.0
+    grow = np.zeros((N, 2))
+    grow[:, 0] = 2.0 ** (((np.arange(N) % 4000) / (8.0 / share) - 480.0) / 2) * (rng.random(N) < 0.9)
+    tiny = rng.standard_normal((N, 2)) * 1e-153 * (rng.random((N, 2)) < share)
+    for b in (a, grow, tiny):
+        cdf = np.cumsum(terms(b))
+        with tq.GpuState(tq.FP64) as g:
+            g.load(n, b.reshape(-1))
+            assert g.total_probability() == cdf[-1]
+            assert g.amplitude_sum() == (np.cumsum(b[:, 0])[-1], np.cumsum(b[:, 1])[-1])
+            for i in (0, 5, N // 3, N // 2 + 17, N - 1):
+                for r in (cdf[i], np.nextafter(cdf[i], 0), np.nextafter(cdf[i], 2)):
+                    if 0.0 <= r < 1.0 and r <= cdf[-1]:
+                        assert g.sample(float(r)) == int(np.argmax(r <= cdf))
