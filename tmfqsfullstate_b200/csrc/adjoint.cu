@@ -373,11 +373,11 @@ unsigned launch_obs_apply(const LaunchCtx &c, int prec, const void *psi, void *l
 	const unsigned nbytes = (n + 7) / 8;
 	const size_t smem = sizeof(uint64_t) * 256 * nbytes + sizeof(double) * 256 * ((nterms + 7) / 8);
 	if(prec == TMFQS_FP64) {
-		allow_dynamic_smem(k_obs_apply<double>, "observable smem");
+		allow_dynamic_smem(k_obs_apply<double>, "observable smem", 64);
 		k_obs_apply<double><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<const double2 *>(psi), static_cast<double2 *>(lam), N, p,
 		                                                              nbytes, dev_partials);
 	} else {
-		allow_dynamic_smem(k_obs_apply<float>, "observable smem");
+		allow_dynamic_smem(k_obs_apply<float>, "observable smem", 64);
 		k_obs_apply<float><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<const float2 *>(psi), static_cast<float2 *>(lam), N, p,
 		                                                             nbytes, dev_partials);
 	}
@@ -423,12 +423,12 @@ unsigned launch_grad_run(const LaunchCtx &c, int prec, void *lam, void *psi, uns
 	const unsigned nbytes = (n + 7) / 8;
 	if(prec == TMFQS_FP64) {
 		const size_t smem = grad_smem(sizeof(double), sizeof(double2), nbytes);
-		allow_dynamic_smem(k_grad_run<double, double>, "gradient smem");
+		allow_dynamic_smem(k_grad_run<double, double>, "gradient smem", 64);
 		k_grad_run<double, double><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<double2 *>(lam), static_cast<double2 *>(psi), N, rp,
 		                                                                    nbytes, up, shares, dev_partials);
 	} else {
 		const size_t smem = grad_smem(sizeof(float), sizeof(float2), nbytes);
-		allow_dynamic_smem(k_grad_run<float, float>, "gradient smem");
+		allow_dynamic_smem(k_grad_run<float, float>, "gradient smem", 64);
 		k_grad_run<float, float><<<blocks, kAdjThreads, smem, c.stream>>>(static_cast<float2 *>(lam), static_cast<float2 *>(psi), N, rp,
 		                                                                  nbytes, up, shares, dev_partials);
 	}

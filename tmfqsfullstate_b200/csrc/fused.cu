@@ -875,7 +875,7 @@ void run_fused(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_pr
 	if(!maps.empty()) std::memcpy(host.data() + map_off, maps.data(), maps.size() * sizeof(ChainMap));
 	upload_async(c, dev_prog, host.data(), need, "fused program upload");
 	const size_t smem = (sizeof(typename Vec2<R>::type) << pass.K) + (sizeof(uint64_t) << (pass.K - g.m));
-	allow_dynamic_smem(k_fused<R>, "fused smem");
+	allow_dynamic_smem(k_fused<R>, "fused smem", 6 * 1024);
 	int per_sm = 1;
 	check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<R>, kFusedThreads, smem), "fused occupancy");
 	const uint64_t grid = std::min<uint64_t>(g.ntiles - g.o_begin, (uint64_t)c.num_sms * std::max(1, per_sm));

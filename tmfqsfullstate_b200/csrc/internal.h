@@ -25,20 +25,14 @@ struct Error {
 [[noreturn]] void fail(int status, const std::string &message);
 void check_cuda(cudaError_t e, const char *what);
 
-// Lets a kernel take any dynamic shared memory that its static part leaves.  The
-// same limit whatever the launch needs: the limit belongs to the kernel, and one
-// of each launch's own size was lowered by another thread's between here and the
-// launch, which then failed.
+// Lets a kernel take any dynamic shared memory that its static part (at most
+// `static_bytes`) leaves.  The same limit whatever the launch needs: the limit
+// belongs to the kernel, and one of each launch's own size was lowered by another
+// thread's between here and the launch, which then failed.
+constexpr int kMaxSmem = 227 * 1024;  // of a block, sm_100
 template <typename K>
-void allow_dynamic_smem(K kern, const char *what) {
-	cudaFuncAttributes at;
-	int dev = 0, optin = 0;
-	check_cuda(cudaFuncGetAttributes(&at, kern), what);
-	check_cuda(cudaGetDevice(&dev), what);
-	check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), what);
-	const int limit = optin - (int)at.sharedSizeBytes;
-	if(at.maxDynamicSharedSizeBytes != limit)
-		check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit), what);
+void allow_dynamic_smem(K kern, const char *what, int static_bytes = 0) {
+	check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - static_bytes), what);
 }
 
 // cudaMalloc for the library's device buffers.  While the failure knob of

@@ -888,7 +888,7 @@ bool run_radix(const LaunchCtx &c, void *a, const FusedPass &pass, void *&dev_pr
 	}
 
 	const unsigned threads = 1u << (K - RB);
-	allow_dynamic_smem(k_radix<R, RB>, "radix smem");
+	allow_dynamic_smem(k_radix<R, RB>, "radix smem", 64);
 	const uint64_t grid = std::min<uint64_t>(P.g.ntiles, (uint64_t)c.num_sms);
 	k_radix<R, RB><<<(unsigned)grid, threads, smem, c.stream>>>(static_cast<V *>(a), P.g,
 	                                                           static_cast<const unsigned char *>(dev_prog), o_st, o_it,
