@@ -45,9 +45,9 @@ constexpr unsigned kMaxRB = 5;
 constexpr unsigned kMaxK = 13;
 constexpr unsigned kMaxStages = 64;
 constexpr unsigned kMaxOps = 240;
-// Fast forms: the Hadamards whose 1/sqrt(2) is outstanding at one time, as in the
-// radix passes on a tile.  (240 of them would be 2^120: a complex64 register that
-// is not normalised overflowed from values of 10^3 on.)
+// Fast forms: the Hadamards whose 1/sqrt(2) is outstanding at one time: values stay
+// within 2^6 of their true size.  (240 of them would be 2^120: a complex64 register
+// that is not normalised overflowed from values of 10^3 on.)
 constexpr unsigned kMaxDeferred = 12;
 
 // Tiles of 64 KiB.
@@ -93,6 +93,10 @@ constexpr unsigned kCodeH = 0, kCodeX = 5, kCodeCP = 30, kCodeScale = kCodeCP + 
 // per launch (entry 0: all amplitudes, 1 + i: those with register bit i), and
 // one that depends on the tile, formed once per tile (the same entries, then
 // 6 + k: for threads with thread bit k).  Both are products in FP64, rounded once.
+// Against the radix stages, 24 qubits: 4, 6 and 12 phases behind four Hadamards 128,
+// 129 and 131 us, there 178, 180 and 184 (2 and 3 phases 164 and 175 in both); a ring of
+// 24 phases with 8, 16 and 24 more on register bits 169, 200 and 232 us, there 211, 215
+// and 218 (14 qubits: 38, 42 and 46; 45, 49 and 52).
 constexpr unsigned kMaxLoose = 8;
 constexpr unsigned kMaxDiag = 2, kDiagMin = 6, kDiagThread = 6, kDiagTile = 6 + 8;
 
